@@ -243,6 +243,18 @@ def run_reference_arm(args):
     d.close()
 
 
+def step_launches(kdesc, steps):
+    """Launches of the library's kernels for one timed call of `steps` steps:
+    the persistent kernel takes 64 steps at a time, each time after its reset
+    kernel (an odd rest of a two-step order separately); the other step
+    kernels are launched per step, twice where planes carry link masks."""
+    if "persist_batch_kernel" not in kdesc:
+        return steps * (2 if "links_pass_kernel" in kdesc else 1)
+    full, rest = divmod(steps, 64)
+    extra = (2 if rest > 2 and rest % 2 and "2 steps per sweep" in kdesc else 1) if rest else 0
+    return 2 * (full + extra)
+
+
 def parity_fracs(bpc, cells, ms_even, ms_odd, n_even, n_odd, peak):
     """Roofline fraction of the even- and odd-parity step launches (mean
     launch time of each)."""
@@ -380,9 +392,9 @@ def run_ours(args):
     tot, _, _ = ch.step_timed(args.steps, per_launch=False)
     clk.stop()
     tmax = d.max(tot)
-    # the device time of every launch comes from a second run of K steps with
-    # an event pair around each launch; events between launches keep a launch
-    # from overlapping the end of the one before, so that run is not `value`
+    # the device time of each parity comes from a second run of K steps, one
+    # step per launch with an event pair around each: a step that does not
+    # overlap the next and finds nothing of it in L2, so that run is not `value`
     _, even, odd = ch.step_timed(args.steps)
     n_even = (args.steps + 1) // 2 if (args.warmup + args.steps) % 2 == 0 else args.steps // 2
     n_odd = args.steps - n_even
@@ -499,7 +511,7 @@ def run_ours(args):
                            "parallelism": f"replicas x{d.world}" if d.world > 1 else "single GPU",
                            "l2": f"state {cells * 19 * args.precision / 8 / 1e9:.2f} GB vs 126 MB L2, no flush"},
                 "variants": variants, "roofline": roof, "e2e": e2e, "cpu_baseline": cb,
-                "gpu_launches": args.steps * (2 if "links_pass_kernel" in kdesc else 1), "clocks": clk.summary()}
+                "gpu_launches": step_launches(kdesc, args.steps), "clocks": clk.summary()}
         # short summaries last, so that a reader of the line's tail sees them
         if batched is not None:
             line["batched"] = batched_summary(batched)

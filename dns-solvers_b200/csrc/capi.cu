@@ -33,27 +33,49 @@ cudaError_t launch_correlations(const double *vel, int nx, int ny, int zd, int p
 size_t spectra_scratch(int nx, int ny, int zd, int jb);
 cudaError_t launch_spectra(const double *vel, int nx, int ny, int zd, int jb, double *scratch, double *ex, double *ey,
                            cudaStream_t s);
-int persist_prepare_f64(size_t smem);
-int persist_occupancy_f64(int threads, size_t smem, bool any_q);
-cudaError_t launch_persist_f64(const PersistArgs &a, int grid, int threads, size_t smem, bool any_q, cudaStream_t s);
-int persist_prepare_lp(int precision, size_t smem);
-int persist_occupancy_lp(int precision, int threads, size_t smem, bool any_q);
-cudaError_t launch_persist_lp(int precision, const PersistArgs &a, int grid, int threads, size_t smem, bool any_q,
-                              cudaStream_t s);
-static int persist_prepare(int precision, size_t smem)
+#define DNSLBM_PERSIST_DECL(S)                                                                                      \
+    int persist_prepare_##S(int threads, size_t smem, bool any_q, bool links);                                                                          \
+    int persist_occupancy_##S(int threads, size_t smem, bool any_q, bool links);                                   \
+    cudaError_t launch_persist_##S(const PersistArgs &a, unsigned groups, int grid, int threads, size_t smem,      \
+                                   bool any_q, bool links, cudaStream_t s);
+DNSLBM_PERSIST_DECL(f64)
+DNSLBM_PERSIST_DECL(f32)
+DNSLBM_PERSIST_DECL(f16)
+DNSLBM_PERSIST_DECL(batch_f64)
+DNSLBM_PERSIST_DECL(batch_f32)
+DNSLBM_PERSIST_DECL(batch_f16)
+#undef DNSLBM_PERSIST_DECL
+// batch: the form that reads a launch table, else the form of one channel
+static int persist_prepare(int precision, bool batch, int threads, size_t smem, bool any_q, bool links)
 {
-    return precision == 64 ? persist_prepare_f64(smem) : persist_prepare_lp(precision, smem);
+    if (batch)
+        return precision == 64   ? persist_prepare_batch_f64(threads, smem, any_q, links)
+               : precision == 32 ? persist_prepare_batch_f32(threads, smem, any_q, links)
+                                 : persist_prepare_batch_f16(threads, smem, any_q, links);
+    return precision == 64   ? persist_prepare_f64(threads, smem, any_q, links)
+           : precision == 32 ? persist_prepare_f32(threads, smem, any_q, links)
+                             : persist_prepare_f16(threads, smem, any_q, links);
 }
-static int persist_occupancy_of(int precision, int threads, size_t smem, bool any_q)
+static int persist_occupancy_of(int precision, bool batch, int threads, size_t smem, bool any_q, bool links)
 {
-    return precision == 64 ? persist_occupancy_f64(threads, smem, any_q)
-                           : persist_occupancy_lp(precision, threads, smem, any_q);
+    if (batch)
+        return precision == 64   ? persist_occupancy_batch_f64(threads, smem, any_q, links)
+               : precision == 32 ? persist_occupancy_batch_f32(threads, smem, any_q, links)
+                                 : persist_occupancy_batch_f16(threads, smem, any_q, links);
+    return precision == 64   ? persist_occupancy_f64(threads, smem, any_q, links)
+           : precision == 32 ? persist_occupancy_f32(threads, smem, any_q, links)
+                             : persist_occupancy_f16(threads, smem, any_q, links);
 }
-static cudaError_t launch_persist_batch(int precision, const PersistArgs &a, int grid, int threads, size_t smem,
-                                        bool any_q, cudaStream_t s)
+static cudaError_t launch_persist_of(int precision, bool batch, const PersistArgs &a, unsigned groups, int grid, int threads,
+                                     size_t smem, bool any_q, bool links, cudaStream_t s)
 {
-    return precision == 64 ? launch_persist_f64(a, grid, threads, smem, any_q, s)
-                           : launch_persist_lp(precision, a, grid, threads, smem, any_q, s);
+    if (batch)
+        return precision == 64   ? launch_persist_batch_f64(a, groups, grid, threads, smem, any_q, links, s)
+               : precision == 32 ? launch_persist_batch_f32(a, groups, grid, threads, smem, any_q, links, s)
+                                 : launch_persist_batch_f16(a, groups, grid, threads, smem, any_q, links, s);
+    return precision == 64   ? launch_persist_f64(a, groups, grid, threads, smem, any_q, links, s)
+           : precision == 32 ? launch_persist_f32(a, groups, grid, threads, smem, any_q, links, s)
+                             : launch_persist_f16(a, groups, grid, threads, smem, any_q, links, s);
 }
 int tma_prepare_f64(size_t smem);
 int tma_occupancy_f64(int threads, size_t smem, bool const_q);
@@ -90,6 +112,8 @@ struct dnslbm_ctx {
     int *band_of = nullptr;      // [nz] mask block of a plane next to a solid, -1: none
     unsigned *links = nullptr;   // [nband][ny][nx] per-cell link masks
     size_t links_bytes = 0;
+    unsigned long long *link_rows = nullptr;  // [nband][ny] RowInfo
+    size_t link_rows_n = 0;
     int nband = 0;
     // planes of the row-pipelined kernel (nclean, ascending) followed by the
     // planes with link masks (ndirty), which a second launch steps per cell
@@ -98,6 +122,17 @@ struct dnslbm_ctx {
     int nclean = 0, ndirty = 0;
     LinksLaunch *d_llaunch = nullptr;  // the second launch's table (one entry)
     int tma_target = 0;                // resident blocks of the row-pipelined kernel
+    // the persistent time-loop kernel (step_persist.cuh): the memory its
+    // blocks share
+    unsigned *flow_flags = nullptr;   // per row group
+    size_t flow_flags_n = 0;
+    FlowMaps maps = {};               // tensor maps of the populations, for groups of maps_k rows
+    int maps_k = 0, maps_ok = 0;
+    double *flow_part = nullptr;      // [kRing][row groups][NP]
+    size_t flow_part_n = 0;
+    double *flow_sums = nullptr;      // [kRing][nz][NP]
+    unsigned *flow_ctr = nullptr;     // [kRing][nz] groups done, [kRing] planes done, the item counter
+    long long *flow_base = nullptr;
     double *force = nullptr, *shift = nullptr, *partials = nullptr, *plane_sums = nullptr, *logs = nullptr;
     long long *step_ctr = nullptr, *status = nullptr;
     unsigned *plane_ctr = nullptr, *total_ctr = nullptr;
@@ -167,10 +202,22 @@ static int fail(dnslbm_ctx *c, int code, const char *fmt, ...)
         if (e_ != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
+// The context steps with the persistent kernel.
+static bool uses_flow(const dnslbm_ctx *c) { return c->use_tma && !c->slab && c->tma.nseg == 1; }
+
+// Place of population a among the arrays: in groups for the persistent
+// kernel's tensor copies, in the lattice's order otherwise.  A context changes kernels only while it holds no state.
+static int array_pos(const dnslbm_ctx *c, int a) { return uses_flow(c) ? lat_pos(a) : a; }
+
+// Steps that may be in flight at once in the persistent kernel (entries of
+// its per-step sums and of a whole channel's shift array); a power of two,
+// well above the steps of two sweeps (flow_order).
+constexpr int kRing = 8;
+
 static StepArgs step_args(const dnslbm_ctx *c)
 {
     StepArgs p;
-    for (int a = 0; a < Q; ++a) p.pop[a] = (char *)c->popmem + ((size_t)a * c->pstride + c->pop_off) * c->esize;
+    for (int a = 0; a < Q; ++a) p.pop[a] = (char *)c->popmem + ((size_t)array_pos(c, a) * c->pstride + c->pop_off) * c->esize;
     p.nx = c->nx;
     p.ny = c->ny;
     p.nz = c->nz;
@@ -194,18 +241,36 @@ static StepArgs step_args(const dnslbm_ctx *c)
     p.status = c->status;
     p.band_of = c->band_of;
     p.links = c->links;
+    p.link_rows = c->link_rows;
     p.wait_ns = c->wait_ns;
     p.withhold_stage = 0;
     p.wall_lo = c->wall_lo;
     p.wall_hi = c->wall_hi;
     p.tail = c->slab ? 0 : 1;
+    p.ring = c->slab ? 0 : kRing;
     return p;
 }
+
+// Rows that divide into equal pieces of whole 16 bytes and at most 256 words
+// of 8 bytes (the pieces, 0: they do not), and whose groups of k fill whole
+// 128 bytes: what the tensor maps need.
+static int row_pieces(size_t row_bytes)
+{
+    const size_t words = row_bytes / 8;
+    for (size_t n = (words + 255) / 256; row_bytes % 16 == 0 && n <= 16; ++n)
+        if (words % n == 0 && words / n % 2 == 0) return (int)n;
+    return 0;
+}
+
+static bool tensor_rows(size_t row_bytes, int k) { return row_pieces(row_bytes) > 0 && row_bytes * k % 128 == 0; }
+
+static size_t shift_bytes(const dnslbm_ctx *c) { return (size_t)(c->slab ? 2 : kRing) * c->nz * 3 * sizeof(double); }
+static size_t flow_ctr_bytes(const dnslbm_ctx *c) { return ((size_t)kRing * (c->nz + 1) + 1) * sizeof(unsigned); }
 
 static IoArgs io_args(const dnslbm_ctx *c)
 {
     IoArgs p;
-    for (int a = 0; a < Q; ++a) p.pop[a] = (char *)c->popmem + ((size_t)a * c->pstride + c->pop_off) * c->esize;
+    for (int a = 0; a < Q; ++a) p.pop[a] = (char *)c->popmem + ((size_t)array_pos(c, a) * c->pstride + c->pop_off) * c->esize;
     p.nx = c->nx;
     p.ny = c->ny;
     p.nz = c->nz;
@@ -225,7 +290,8 @@ static void free_all(dnslbm_ctx *c)
                     c->total_ctr,  c->staging,    c->stat_partials, c->stat_planes, c->stat_mean,
                     c->band_of,    c->links,      c->plane_list,    c->d_llaunch,   c->stat_acc,
                     c->out_lbf,    c->out_vel,    c->out_den,       c->out_stats,   c->quad_buf,
-                    c->shift_all};
+                    c->shift_all,  c->flow_flags,    c->flow_part,   c->flow_sums,
+                    c->flow_ctr,   c->flow_base,  c->link_rows};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (auto &e : c->ev)
@@ -276,8 +342,8 @@ constexpr int kMaxSegments = 4;
 static int tma_configure(dnslbm_ctx *c, int k, int stages, int consumers, int bps, int seg = 0)
 {
     const int row_bytes = c->pitch * (int)c->esize;
-    k = std::max(1, std::min(k, c->ny));
-    consumers = std::max(32, std::min(352, consumers / 32 * 32));
+    k = std::max(1, std::min(std::min(k, c->ny), kMaxGroupRows));
+    consumers = std::max(32, std::min(c->slab || seg > 0 ? 352 : 32 * kMaxConsumerWarps, consumers / 32 * 32));
     if (seg > 0 && (c->deck.precision != 64 || seg % 2 || seg >= c->nx)) return -1;
     if (seg > 0) k = 1;
     const int nseg = seg > 0 ? (c->nx + seg - 1) / seg : 1;
@@ -287,17 +353,29 @@ static int tma_configure(dnslbm_ctx *c, int k, int stages, int consumers, int bp
     int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->deck.device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->deck.device);
-    const size_t smem = (size_t)stages * smem_stage + 16 * (size_t)stages;  // + full/empty mbarriers
+    // whole channels step with the persistent kernel (two special warps);
+    // slabs, and rows in x-segments, with one launch per step (one producer
+    // warp: 1256x157x100 FP64 1133 us/step against 1217 in the persistent
+    // kernel, whose stages wait longer for the edge cells' loads)
+    const bool per_step = c->slab || seg > 0;
+    const size_t smem = per_step ? (size_t)stages * smem_stage + 16 * (size_t)stages : persist_smem(stages, smem_stage);
     const size_t cap = (size_t)maxsmem - kStaticSmemReserve;  // room for the kernels' static shared memory
     if (stages < 2 || smem > cap || nsm <= 0) return -1;
-    const int threads = consumers + 32;
+    const int threads = consumers + (per_step ? 32 : 64);
     const bool const_q = c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
-    // the kernels may use up to the device's opt-in shared memory (a batch can
-    // give a channel a larger stage than its own shape)
-    const int prep = c->deck.precision == 64 ? tma_prepare_f64(cap) : tma_prepare_lp(c->deck.precision, cap);
-    int occ = prep ? 0
-                   : (c->deck.precision == 64 ? tma_occupancy_f64(threads, smem, const_q)
-                                              : tma_occupancy_lp(c->deck.precision, threads, smem, const_q));
+    int occ = 0;
+    if (per_step) {
+        const int prep = c->deck.precision == 64 ? tma_prepare_f64(cap) : tma_prepare_lp(c->deck.precision, cap);
+        if (!prep)
+            occ = c->deck.precision == 64 ? tma_occupancy_f64(threads, smem, const_q)
+                                          : tma_occupancy_lp(c->deck.precision, threads, smem, const_q);
+    } else {
+        // with solids inside the flow the flags decide which form runs
+        const bool general = c->deck.bc_mode == DNSLBM_BC_GENERAL;
+        int prep = persist_prepare(c->deck.precision, false, threads, cap, const_q, false);
+        if (!prep && general) prep = persist_prepare(c->deck.precision, false, threads, cap, const_q, true);
+        if (!prep) occ = persist_occupancy_of(c->deck.precision, false, threads, smem, const_q, general);
+    }
     cudaGetLastError();  // a failed query only rules the configuration out
     if (bps > 0) occ = std::min(occ, bps);
     if (occ < 1) return -1;
@@ -315,9 +393,46 @@ static int tma_configure(dnslbm_ctx *c, int k, int stages, int consumers, int bp
 // x-segment length (even) that splits rows of nx into nseg near-equal parts.
 static int segment_for(int nx, int nseg) { return ((nx + nseg - 1) / nseg + 1) & ~1; }
 
+// The order of a channel's items in the persistent kernel for `blocks`
+// resident blocks: how many steps run through it at once, and their distance
+// in row groups.
+struct FlowOrder {
+    int depth, lag;
+};
+
+// Two steps at once where the state does not stay in L2 (126 MB) by itself
+// and what the second step needs of the first does: of what a step reads,
+// the second finds most in L2.  The distance is a plane, because a row's
+// neighbours are in the planes around it, and twice the row groups the
+// blocks hold in their stages, so that a group's neighbours are done when its
+// turn comes (a group is done about 8000 cycles after its collision: its
+// stores land); a shorter distance makes the blocks wait, a longer one loses
+// data from L2.  Measured on a B200, microseconds per step, one step at a
+// time / two / two with a distance of 0.6, 1.25 and 3 times the stages: FP32
+// 628x314x200 993 / 929 / 1421, 980, 970; FP16 515 / 475 / 834, 523, 502;
+// FP64 302x151x96 233 / 205 / -, 223, 223.  Four at once measured slower
+// (FP32 1019, FP16 543).
+// A constant flow rate takes every step's force from the whole state before
+// it: one step at a time.
+static FlowOrder flow_order(const dnslbm_ctx *c, int blocks)
+{
+    const TmaArgs &t = c->tma;
+    const double group_bytes = (double)Q * t.dir_elems * c->esize, groups = (double)t.gpp * c->nz;
+    if (c->deck.force_mode == DNSLBM_FORCE_CONST_Q || groups * group_bytes <= 90e6) return {1, 0};
+    const int lag = t.gpp + 4 + blocks * t.stages;
+    if ((2.0 * lag + t.gpp) * group_bytes > 160e6 || 2.0 * lag > 0.75 * groups) return {1, 0};
+    return {2, lag};
+}
+
 static void describe_kernel(dnslbm_ctx *c)
 {
-    if (c->use_tma) {
+    if (uses_flow(c)) {
+        snprintf(c->kernel_desc, sizeof c->kernel_desc,
+                         "persist_batch_kernel<fp%d> row-pipelined bulk-copy: %d blocks x %d threads, groups of %d rows, "
+                         "%d stages, %zu B smem, %d steps per sweep",
+                         c->deck.precision, c->tma_target, c->tma_threads, c->tma.k, c->tma.stages, c->tma_smem,
+                         flow_order(c, c->tma_target).depth);
+    } else if (c->use_tma) {
         int m = snprintf(c->kernel_desc, sizeof c->kernel_desc,
                          "step_tma_kernel<fp%d> row-pipelined bulk-copy: %d blocks x %d threads, %d groups of %d "
                          "rows/block, %d stages, %zu B smem",
@@ -352,6 +467,20 @@ static cudaError_t upload_planes(dnslbm_ctx *c, const std::vector<int> *band = n
     c->ndirty = c->nz - c->nclean;
     c->plane_host = pl;
     return cudaMemcpy(c->plane_list, pl.data(), pl.size() * sizeof(int), cudaMemcpyHostToDevice);
+}
+
+// Default rows per stage group.  FP32 with a constant flow rate keeps powers of
+// two (and its consumer count): its FP32 partial sums, and through the force
+// the state's roundings, depend on which cells a thread sums.
+static int default_rows(const dnslbm_ctx *c, size_t row_bytes)
+{
+    const size_t most = c->slab && c->deck.precision == 16 ? 49152 : 98304;
+    int k = 1;
+    if (c->slab || (c->deck.precision != 64 && c->deck.force_mode == DNSLBM_FORCE_CONST_Q))
+        while (k < 8 && k * 2 <= c->ny && (size_t)Q * row_bytes * k * 2 <= most) k *= 2;
+    else
+        while (k < 8 && k + 1 <= c->ny && (size_t)Q * row_bytes * (k + 1) <= most) ++k;
+    return k;
 }
 
 // A whole channel (slab = 0) or the wall-normal slab [z0, z0 + nzs) of one
@@ -403,9 +532,18 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         // not 632 elements), FP16 faster on 32 bytes (640, not 632); FP64
         // rows of 628 are 32-byte multiples either way.
         int align_bytes = c->esize == 4 ? 16 : 32;
-        if (const char *e = getenv("DNSLBM_ROW_ALIGN")) align_bytes = std::max(16, atoi(e));
+        const char *e = getenv("DNSLBM_ROW_ALIGN");
+        if (e) align_bytes = std::max(16, atoi(e));
         const int v = align_bytes / (int)c->esize;
         c->pitch = (c->nx + v - 1) / v * v;
+        if (!slab && !e && (size_t)2 * Q * c->pitch * c->esize <= (size_t)216 * 1024) {  // two whole-row stages fit
+            // rows that tensor copies can move in groups of the default size
+            // (tensor_rows): up to 5 % longer
+            size_t row = (size_t)c->pitch * c->esize;
+            const size_t most = row + row / 20;
+            while (row <= most && !tensor_rows(row, default_rows(c, row))) row += 16;
+            if (row <= most) c->pitch = (int)(row / c->esize);
+        }
     }
     c->ncell = (size_t)c->pitch * c->ny * c->nz;
     const size_t align = 256 / c->esize;
@@ -448,14 +586,15 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         // choices; the DNSLBM_* environment variables override them.
         const char *path = getenv("DNSLBM_PATH");
         const int row_bytes = c->pitch * (int)c->esize;
-        const size_t stage_target = c->deck.precision == 16 ? 49152 : 98304;
-        int k = 1;
-        while (k < 8 && k * 2 <= c->ny && (size_t)Q * row_bytes * k * 2 <= stage_target) k *= 2;
+        int k = default_rows(c, row_bytes);
         if (const char *e = getenv("DNSLBM_GROUP_ROWS")) k = std::max(1, std::min(atoi(e), c->ny));
         int stages = 2;
         if (const char *e = getenv("DNSLBM_STAGES")) stages = atoi(e);
-        const int cap = c->deck.precision == 64 ? 320 : (c->deck.precision == 32 ? 192 : 128);
-        int consumers = std::min(cap, (c->nx + 31) / 32 * 32);
+        // consumers: one per cell (FP64) or cell pair of a group, at most 320
+        const bool sums32 = c->deck.precision == 32 && c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
+        const int cap = slab && c->deck.precision == 16 ? 128 : ((slab || sums32) && c->deck.precision == 32 ? 192 : 320);
+        const int cells = slab || sums32 ? c->nx : (k * c->nx + (c->deck.precision != 64)) / (c->deck.precision == 64 ? 1 : 2);
+        int consumers = std::min(cap, (cells + 31) / 32 * 32);
         if (const char *e = getenv("DNSLBM_THREADS")) consumers = atoi(e) / 32 * 32;
         int bps = 0;
         if (const char *e = getenv("DNSLBM_BLOCKS_PER_SM")) bps = atoi(e);
@@ -485,7 +624,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         {&c->popmem, (size_t)Q * c->pstride * c->esize},
         {(void **)&c->wallmask, (size_t)2 * c->nx * c->ny},
         {(void **)&c->force, 2 * sizeof(double)},
-        {(void **)&c->shift, (size_t)2 * c->nz * 3 * sizeof(double)},
+        {(void **)&c->shift, shift_bytes(c)},
         {(void **)&c->partials, nblocks * NP * sizeof(double)},
         {(void **)&c->plane_sums, (size_t)c->nz * NP * sizeof(double)},
         {(void **)&c->logs, (size_t)c->deck.log_capacity * 9 * sizeof(double)},
@@ -501,6 +640,9 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         {(void **)&c->plane_list, (size_t)c->nz * sizeof(int)},
         {(void **)&c->stat_acc, (size_t)9 * c->nz * sizeof(double)},
         {(void **)&c->d_llaunch, sizeof(LinksLaunch)},
+        {(void **)&c->flow_sums, (size_t)kRing * c->nz * NP * sizeof(double)},
+        {(void **)&c->flow_ctr, flow_ctr_bytes(c)},
+        {(void **)&c->flow_base, sizeof(long long)},
     };
     for (auto &a : al) {
         cudaError_t e = cudaMalloc(a.p, a.bytes);
@@ -686,6 +828,31 @@ extern "C" int dnslbm_link_masks(int xdv, int ydv, int zdv, int bc_mode, const i
     return DNSLBM_OK;
 }
 
+// RowInfo of every row of the planes with link masks.
+static std::vector<unsigned long long> link_row_table(int nx, int ny, int nz, const std::vector<int> &band,
+                                                      const std::vector<unsigned> &lk, int nband)
+{
+    std::vector<unsigned long long> rows((size_t)nband * ny, 0ull);
+    for (int z = 0; z < nz; ++z) {
+        if (band[z] < 0) continue;
+        for (int y = 0; y < ny; ++y) {
+            const unsigned *m = &lk[((size_t)band[z] * ny + y) * nx];
+            bool alike = true;
+            for (int x = 1; x < nx && alike; ++x) alike = m[x] == m[0];
+            if (!alike) continue;
+            unsigned long long r = RowInfo::kAlike;
+            if (m[0] & 1u) r |= RowInfo::kSolid;
+            for (int a = 1; a < Q; ++a) {
+                const bool to_wall = (lat_ez(a) < 0 && z == 0) || (lat_ez(a) > 0 && z == nz - 1);
+                const unsigned long long link = (m[0] >> a) & 1u ? 1 : (to_wall ? 2 : 0);
+                r |= link << (2 * a);
+            }
+            rows[(size_t)band[z] * ny + y] = r;
+        }
+    }
+    return rows;
+}
+
 static int apply_flags(dnslbm_ctx *c, const int8_t *fl /* [nx][ny][zd] */)
 {
     const int nx = c->nx, ny = c->ny, nz = c->nz;
@@ -727,6 +894,17 @@ static int apply_flags(dnslbm_ctx *c, const int8_t *fl /* [nx][ny][zd] */)
         if (e != cudaSuccess) return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes of link masks failed", lbytes);
         c->links_bytes = lbytes;
     }
+    const std::vector<unsigned long long> rows = link_row_table(nx, ny, nz, band, lk, nband);
+    if (rows.size() > c->link_rows_n) {
+        if (c->link_rows) CK(cudaFree(c->link_rows));
+        c->link_rows = nullptr;
+        c->link_rows_n = 0;
+        cudaError_t e = cudaMalloc((void **)&c->link_rows, rows.size() * sizeof rows[0]);
+        if (e != cudaSuccess) return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes of link rows failed", rows.size() * sizeof rows[0]);
+        c->link_rows_n = rows.size();
+    }
+    if (!rows.empty())
+        CK(cudaMemcpyAsync(c->link_rows, rows.data(), rows.size() * sizeof rows[0], cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->wallmask, m.data(), m.size(), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->band_of, band.data(), band.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     if (lbytes) CK(cudaMemcpyAsync(c->links, lk.data(), lbytes, cudaMemcpyHostToDevice, c->stream));
@@ -798,7 +976,8 @@ static int reset_counters(dnslbm_ctx *c)
     CK(cudaMemsetAsync(c->total_ctr, 0, sizeof(unsigned), c->stream));
     CK(cudaMemsetAsync(c->step_ctr, 0, sizeof(long long), c->stream));
     CK(cudaMemsetAsync(c->status, 0, 2 * sizeof(long long), c->stream));
-    CK(cudaMemsetAsync(c->shift, 0, (size_t)2 * c->nz * 3 * sizeof(double), c->stream));
+    CK(cudaMemsetAsync(c->shift, 0, shift_bytes(c), c->stream));
+    CK(cudaMemsetAsync(c->flow_ctr, 0, flow_ctr_bytes(c), c->stream));
     if (c->shift_all) CK(cudaMemsetAsync(c->shift_all, 0, (size_t)2 * c->nz_all * 3 * sizeof(double), c->stream));
     c->done = 0;
     c->odd = 0;
@@ -903,8 +1082,135 @@ extern "C" int dnslbm_store_state(dnslbm_ctx *c, double *state)
     return DNSLBM_OK;
 }
 
+// The memory the persistent kernel needs for the channel's row groups.
+static int flow_reserve(dnslbm_ctx *c)
+{
+    const size_t groups = (size_t)c->tma.gpp * c->nz, part = (size_t)kRing * groups * NP;
+    if (groups > c->flow_flags_n) {
+        if (c->flow_flags) CK(cudaFree(c->flow_flags));
+        c->flow_flags = nullptr;
+        c->flow_flags_n = 0;
+        if (cudaMalloc((void **)&c->flow_flags, groups * sizeof(unsigned)) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", groups * sizeof(unsigned));
+        }
+        c->flow_flags_n = groups;
+    }
+    if (part > c->flow_part_n) {
+        if (c->flow_part) CK(cudaFree(c->flow_part));
+        c->flow_part = nullptr;
+        c->flow_part_n = 0;
+        if (cudaMalloc((void **)&c->flow_part, part * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", part * sizeof(double));
+        }
+        c->flow_part_n = part;
+    }
+    return DNSLBM_OK;
+}
+
+// The tensor maps of the channel's row groups; maps_ok unless its rows do not
+// fit them (tensor_rows).
+static void flow_maps(dnslbm_ctx *c)
+{
+    const int k = c->tma.k;
+    if (c->maps_k == k) return;
+    c->maps_k = k;
+    c->maps_ok = 0;
+    const size_t row = (size_t)c->pitch * c->esize;
+    if (!tensor_rows(row, k)) return;
+    typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    const cuuint32_t pieces = (cuuint32_t)row_pieces(row), words = (cuuint32_t)(row / 8 / pieces);
+    const cuuint64_t dims[5] = {words, pieces, (cuuint64_t)c->ny, (cuuint64_t)c->nz, Q};
+    const cuuint64_t strides[4] = {words * 8, row, row * c->ny, c->pstride * c->esize};
+    const cuuint32_t step[5] = {1, 1, 1, 1, 1};
+    CUtensorMap *maps[3] = {&c->maps.all, &c->maps.three, &c->maps.one};
+    const cuuint32_t arrays[3] = {Q, 3, 1};
+    for (int i = 0; i < 3; ++i) {
+        const cuuint32_t box[5] = {words, pieces, (cuuint32_t)k, 1, arrays[i]};
+        if (((Encode)fn)(maps[i], CU_TENSOR_MAP_DATA_TYPE_INT64, 5, c->popmem, dims, strides, box, step,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return;
+    }
+    c->maps_ok = 1;
+}
+
+// The channel's entry of a launch of nsteps steps; its items follow `first`.
+static void flow_entry(const dnslbm_ctx *c, FlowOrder o, int nsteps, unsigned first, ChannelLaunch &L)
+{
+    memset((void *)&L, 0, sizeof L);
+    L.p = step_args(c);
+    L.t = c->tma;
+    L.textured = c->walls_textured;
+    L.depth = nsteps % o.depth ? 1 : o.depth;
+    L.lag = L.depth > 1 ? o.lag : 0;
+    L.flow_groups = (unsigned)c->tma.gpp * (unsigned)c->nz;
+    L.item_first = first;
+    L.item_end = first + flow_items(L.depth, L.lag, L.flow_groups, nsteps);
+    L.pop_bytes = c->pstride * c->esize;
+    L.tensor = c->maps_ok;
+    L.flags = c->flow_flags;
+    L.base = c->flow_base;
+    L.fpart = c->flow_part;
+    L.fsums = c->flow_sums;
+    L.fctr = c->flow_ctr;
+    L.ftotal = c->flow_ctr + (size_t)kRing * c->nz;
+}
+
+// Steps per launch: 64, fewer where the item numbers (32 bits) would run out.
+static int flow_chunk(double groups) { return (int)std::max(1.0, std::min(64.0, std::floor(1e9 / groups))); }
+
+// Few items per step for the stages of all blocks: the next step's items wait
+// for the ones just done, so those are announced at once.
+static int flow_eager(double groups, int blocks, int stages) { return groups < 4.0 * blocks * stages; }
+
+static int flow_steps(dnslbm_ctx *c, long n)
+{
+    if (int rc = flow_reserve(c)) return rc;
+    flow_maps(c);
+    const FlowOrder o = flow_order(c, c->tma_target);
+    const unsigned groups = (unsigned)c->tma.gpp * (unsigned)c->nz;
+    int chunk = flow_chunk(groups);
+    if (chunk >= o.depth) chunk -= chunk % o.depth;
+    PersistArgs a{};
+    a.nchan = 1;
+    a.stages = c->tma.stages;
+    a.stage_bytes = (unsigned)((size_t)Q * c->tma.dir_elems * c->esize);
+    a.counter = c->flow_ctr + (size_t)kRing * (c->nz + 1);
+    a.abort = reinterpret_cast<int *>(c->status + 1);
+    a.wait_ns = c->wait_ns;
+    a.eager = flow_eager(groups, c->tma_target, c->tma.stages);
+    while (n > 0) {
+        int m = (int)std::min<long>(n, chunk);
+        if (m > o.depth && m % o.depth) m -= m % o.depth;  // the rest in a launch of its own
+        a.one_maps = c->maps;
+        ChannelLaunch &L = a.one;
+        flow_entry(c, o, m, 0, L);
+        a.nsteps = m;
+        a.withhold = c->withhold;
+        c->withhold = 0;
+        CK(launch_persist_of(c->deck.precision, false, a, groups, (int)std::min<unsigned>(c->tma_target, L.item_end),
+                                c->tma_threads, c->tma_smem, L.p.const_q != 0, c->ndirty > 0, c->stream));
+        c->odd = (c->odd + m) & 1;
+        c->done += m;
+        n -= m;
+    }
+    return DNSLBM_OK;
+}
+
 static int launch_steps(dnslbm_ctx *c, long n, bool timed, double *ms_even, double *ms_odd)
 {
+    if (uses_flow(c) && !timed) return flow_steps(c, n);
     StepArgs p = step_args(c);
     // timed: an event pair around every launch, read after one final sync
     // (no host round trip between launches)
@@ -917,7 +1223,11 @@ static int launch_steps(dnslbm_ctx *c, long n, bool timed, double *ms_even, doub
     for (long s = 0; s < n; ++s) {
         const bool odd = c->odd != 0;
         if (timed) CK(cudaEventRecord(c->tev[2 * s], c->stream));
-        if (c->use_tma) {
+        if (uses_flow(c)) {
+            if (int rc = flow_steps(c, 1)) return rc;  // counts the step itself
+            c->odd ^= 1;
+            c->done--;
+        } else if (c->use_tma) {
             if (c->withhold && c->tma.ngroups > 0) {  // test hook, one launch only
                 p.withhold_stage = 1;
                 c->withhold = 0;
@@ -1105,7 +1415,7 @@ extern "C" int dnslbm_set_wait_limit(dnslbm_ctx *c, double ms)
 extern "C" int dnslbm_test_withhold_load(dnslbm_ctx *c)
 {
     if (!c) return fail(c, DNSLBM_ERR_ARG, "null context");
-    if (!c->use_tma || c->tma.ngroups <= 0)
+    if (!c->use_tma)
         return fail(c, DNSLBM_ERR_STATE, "the context steps with a kernel that has no bounded waits");
     c->withhold = 1;
     return DNSLBM_OK;
@@ -1621,6 +1931,19 @@ static int time_choice(dnslbm_ctx *c, int steps, double *ms, double *ms_even = n
     CK(cudaGetLastError());
     if ((rc = initial_reduce(c))) return rc;
     double e = 0, o = 0;
+    if (uses_flow(c)) {  // the persistent kernel runs its steps together
+        if ((rc = launch_steps(c, 4, false, nullptr, nullptr))) return rc;
+        CK(cudaEventRecord(c->ev[0], c->stream));
+        if ((rc = launch_steps(c, steps, false, nullptr, nullptr))) return rc;
+        CK(cudaEventRecord(c->ev[1], c->stream));
+        if ((rc = check_status(c))) return rc;
+        float t = 0.f;
+        CK(cudaEventElapsedTime(&t, c->ev[0], c->ev[1]));
+        *ms = t / steps;
+        if (ms_even) *ms_even = *ms;
+        if (ms_odd) *ms_odd = *ms;
+        return DNSLBM_OK;
+    }
     if ((rc = launch_steps(c, 2, true, &e, &o))) return rc;
     e = o = 0;
     if ((rc = launch_steps(c, steps, true, &e, &o))) return rc;
@@ -1715,7 +2038,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
         }
     }
     if (bt.k > 0 && bt.ms < best_ms) best_ms = bt.ms, best = bt.ch;  // one shape for both parities
-    if (be.k > 0) {
+    if (be.k > 0 && (c->slab || be.seg > 0) && (c->slab || bo.seg > 0)) {
         const bool same = be.ch.threads == bo.ch.threads && be.ch.grid == bo.ch.grid && be.ch.smem == bo.ch.smem &&
                           be.ch.t.k == bo.ch.t.k && be.ch.t.stages == bo.ch.t.stages && be.ch.t.nseg == bo.ch.t.nseg;
         if (!same) {  // the parities' own shapes, measured together (a change of shape between launches costs too)
@@ -1751,19 +2074,20 @@ struct dnslbm_batch {
     size_t smem = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // a chunk of steps starting on an even / odd parity
     int graph_steps = 32;
-    // the persistent kernel (default): one cooperative launch per chunk of
-    // steps, blocks taking items of work from a per-step counter
+    // the persistent kernel (default): one launch per chunk of steps,
+    // replayed from a CUDA graph
     int persistent = 1;
     int any_q = 0;                      // some channel runs with a constant flow rate
-    int pgrid = 0;                      // its blocks (all resident)
+    int pgrid = 0;                      // its blocks
     size_t pstage = 0, psmem = 0;       // bytes of one stage, dynamic shared memory
-    std::vector<BatchItem> items;       // the items of one step, largest first
-    int items_per_block = 4;            // items per resident block and step the items are cut for
-    std::vector<BatchItem> items_uploaded;
-    BatchItem *d_items = nullptr;
-    size_t d_items_cap = 0;
-    unsigned *d_counters = nullptr;     // [graph_steps] items taken per step
-    unsigned *d_arrivals = nullptr;     // grid-barrier arrivals
+    int general = 0;                    // some channel may have planes with link masks
+    int any_links = 0;                  // some channel has planes with link masks
+    ChannelLaunch *d_flow = nullptr;    // [2][n] the launch tables of a full chunk and of what is left of a call
+    std::vector<ChannelLaunch> flow_host[2];  // what d_flow holds
+    FlowMaps *d_maps = nullptr;         // [n] the channels' tensor maps
+    std::vector<int> maps_k;            // rows of the groups they are for
+    unsigned groups = 0;                // row groups of all channels
+    unsigned *d_counter = nullptr;      // items taken
     int *d_abort = nullptr;             // a bounded wait of the launch gave up
     int graph_ok = 1;                   // 0: stream capture of the cooperative launch was refused
     int withhold = 0;                   // test hook: the next run withholds a load
@@ -1814,9 +2138,9 @@ extern "C" void dnslbm_batch_destroy(dnslbm_batch *b)
         if (e) cudaEventDestroy(e);
     if (b->d_launch) cudaFree(b->d_launch);
     if (b->d_links) cudaFree(b->d_links);
-    if (b->d_items) cudaFree(b->d_items);
-    if (b->d_counters) cudaFree(b->d_counters);
-    if (b->d_arrivals) cudaFree(b->d_arrivals);
+    if (b->d_flow) cudaFree(b->d_flow);
+    if (b->d_maps) cudaFree(b->d_maps);
+    if (b->d_counter) cudaFree(b->d_counter);
     if (b->d_abort) cudaFree(b->d_abort);
     for (auto &e : b->fj)
         if (e) cudaEventDestroy(e);
@@ -1829,15 +2153,13 @@ extern "C" void dnslbm_batch_destroy(dnslbm_batch *b)
 // Shared-memory budgets per block for one, two and three blocks per SM
 // (228 KB per SM, 1 KB of it reserved per block, the static shared memory of
 // the kernel on top).
-constexpr size_t kBatchBudget1 = 220 * 1024, kBatchBudget2 = 108 * 1024, kBatchBudget3 = 70 * 1024;
+constexpr size_t kBatchBudget1 = 220 * 1024, kBatchBudget2 = 112 * 1024, kBatchBudget3 = 70 * 1024;
 
 // Row groups of every channel's planes without link masks shared among the
 // resident blocks, each block taking whole row groups of one channel and
 // about the same number of cells, and the block count of the per-cell pass
 // over the planes with link masks.  A change of
 // either grid invalidates the captured graphs.
-static void persist_items(dnslbm_batch *b);
-
 static void batch_layout(dnslbm_batch *b)
 {
     // a common amount of work per block (cells of whole row groups), the
@@ -1877,52 +2199,8 @@ static void batch_layout(dnslbm_batch *b)
     b->grid = grid;
     b->links_blocks = lblocks;
     b->nlinks = nl;
-    if (b->persistent) persist_items(b);
-}
-
-// The items of one step of the persistent kernel: each plane of each
-// channel cut into runs of whole row groups of about W cells, W chosen so
-// that every resident block takes about items_per_block items per step (more
-// and smaller items even out the blocks' ends of a step, at a cost per
-// item; the batch autotuner picks the count); kind 1 for the
-// planes with link masks (the channel's plane list holds them after the
-// others, so the group numbering covers them).  Largest first, so the last
-// items taken are the small ones.  An item's slot is its index within its
-// plane, so the plane sums do not depend on which block takes it.
-static void persist_items(dnslbm_batch *b)
-{
-    double total = 0;
-    for (auto *c : b->ch) total += (double)c->nx * c->ny * c->nz;
-    const double W = std::max(1.0, total / ((double)b->items_per_block * std::max(1, b->pgrid)));
-    std::vector<BatchItem> it;
-    std::vector<double> cells;
-    for (int ci = 0; ci < (int)b->ch.size(); ++ci) {
-        dnslbm_ctx *c = b->ch[ci];
-        const TmaArgs &t = c->tma;
-        for (int pi = 0; pi < c->nz; ++pi) {
-            const double gcells = (double)t.k * c->nx;
-            const int per = std::max(1, (int)(W / gcells));
-            const int n = (t.gpp + per - 1) / per;
-            for (int j = 0; j < n; ++j) {
-                const int g0 = (int)((long long)t.gpp * j / n), g1 = (int)((long long)t.gpp * (j + 1) / n);
-                BatchItem x{};
-                x.chan = ci;
-                x.kind = pi < c->nclean ? 0 : 1;
-                x.first = pi * t.gpp + g0;
-                x.count = g1 - g0;
-                x.plane = c->plane_host[pi];
-                x.slot = j;
-                x.ncontrib = n;
-                it.push_back(x);
-                cells.push_back(std::min((double)(g1 - g0) * t.k, (double)c->ny) * c->nx);
-            }
-        }
-    }
-    std::vector<int> order(it.size());
-    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cells[a] > cells[c]; });
-    b->items.resize(it.size());
-    for (size_t i = 0; i < order.size(); ++i) b->items[i] = it[order[i]];
+    if ((nl > 0) != (b->any_links != 0)) destroy_graphs(b);  // another form of the persistent kernel
+    b->any_links = nl > 0;
 }
 
 // Shape of the persistent kernel for the current stages and consumers:
@@ -1931,16 +2209,23 @@ static int persist_configure(dnslbm_batch *b)
 {
     size_t stage = 0;
     for (auto *c : b->ch) stage = std::max(stage, (size_t)Q * c->tma.row_bytes * c->tma.k);
-    const size_t smem = persist_smem(b->stages, stage);
+    stage = (stage + 127) / 128 * 128;  // tensor copies land on 128 bytes
+    const size_t smem = persist_smem(b->stages, stage, (int)b->ch.size());
     int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
     const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
     if (smem > cap || nsm < 1) return -1;
     b->any_q = 0;
-    for (auto *c : b->ch) b->any_q |= c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
-    const int occ =
-        persist_prepare(b->precision, cap) ? 0 : persist_occupancy_of(b->precision, b->threads, smem, b->any_q != 0);
+    b->general = 0;
+    for (auto *c : b->ch) {
+        b->any_q |= c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
+        b->general |= c->deck.bc_mode == DNSLBM_BC_GENERAL;
+    }
+    const int occ = persist_prepare(b->precision, true, b->threads, cap, b->any_q != 0, false) ||
+                            (b->general && persist_prepare(b->precision, true, b->threads, cap, b->any_q != 0, true))
+                        ? 0
+                        : persist_occupancy_of(b->precision, true, b->threads, smem, b->any_q != 0, b->general != 0);
     cudaGetLastError();
     if (occ < 1) return -1;
     b->pstage = stage;
@@ -1956,32 +2241,45 @@ static int persist_configure(dnslbm_batch *b)
 // when it runs on the device.
 static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consumers)
 {
-    consumers = std::max(32, std::min(352, consumers / 32 * 32));
+    const int special = b->persistent ? 64 : 32;  // threads of the load and store warps, or of the producer
+    consumers = std::max(32, std::min(b->persistent ? 32 * kMaxConsumerWarps : 352, consumers / 32 * 32));
     size_t smem = 0;
     std::vector<int> ks(b->ch.size());
     for (size_t i = 0; i < b->ch.size(); ++i) {
         dnslbm_ctx *c = b->ch[i];
         const int row_bytes = c->pitch * (int)c->esize;
-        auto need = [&](int k) { return (size_t)stages * Q * row_bytes * k + 16 * (size_t)stages; };
+        auto need = [&](int k) {
+            return b->persistent ? persist_smem(stages, (size_t)Q * row_bytes * k, (int)b->ch.size())
+                                 : (size_t)stages * Q * row_bytes * k + 16 * (size_t)stages;
+        };
         if (need(1) > budget) return -1;
         int k = 1;
         while (k < 16 && k + 1 <= c->ny && need(k + 1) <= budget) ++k;
+        // a size that tensor copies take, if one is near
+        if (b->persistent)
+            for (int q = k; q >= 1 && 4 * q >= 3 * k; --q)
+                if (tensor_rows((size_t)row_bytes, q)) {
+                    k = q;
+                    break;
+                }
         ks[i] = k;
         smem = std::max(smem, need(k));
     }
-    const int threads = consumers + 32;
-    int maxsmem = 0;
+    const int threads = consumers + special;
+    int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
-    if (smem > cap) return -1;
-    const int prep = b->precision == 64 ? tma_batch_prepare_f64(cap) : tma_batch_prepare_lp(b->precision, cap);
-    const int occ = prep ? 0
-                         : (b->precision == 64 ? tma_batch_occupancy_f64(threads, smem)
-                                               : tma_batch_occupancy_lp(b->precision, threads, smem));
-    cudaGetLastError();  // a failed query only rules the shape out
-    int nsm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
-    if (occ < 1 || nsm < 1) return -1;
+    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
+    if (smem > cap || nsm < 1) return -1;
+    int occ = 1;
+    if (!b->persistent) {
+        const int prep = b->precision == 64 ? tma_batch_prepare_f64(cap) : tma_batch_prepare_lp(b->precision, cap);
+        occ = prep ? 0
+                   : (b->precision == 64 ? tma_batch_occupancy_f64(threads, smem)
+                                         : tma_batch_occupancy_lp(b->precision, threads, smem));
+        cudaGetLastError();  // a failed query only rules the shape out
+        if (occ < 1) return -1;
+    }
     for (size_t i = 0; i < b->ch.size(); ++i) {
         dnslbm_ctx *c = b->ch[i];
         const int row_bytes = c->pitch * (int)c->esize;
@@ -1997,7 +2295,17 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
     b->smem = smem;
     b->budget = budget;
     b->stages = stages;
-    if (b->persistent && persist_configure(b)) return -1;
+    if (b->persistent) {
+        if (persist_configure(b)) return -1;
+        for (auto *c : b->ch) {  // what a channel stepped by itself takes: the same stages, its own stage size
+            c->tma_smem = persist_smem(stages, (size_t)Q * c->tma.dir_elems * c->esize);
+            c->tma_target = b->pgrid;
+            const bool q = c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
+            if (persist_prepare(b->precision, false, threads, cap, q, false) ||
+                (c->deck.bc_mode == DNSLBM_BC_GENERAL && persist_prepare(b->precision, false, threads, cap, q, true)))
+                return -1;
+        }
+    }
     destroy_graphs(b);
     batch_layout(b);
     return 0;
@@ -2041,11 +2349,12 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
         return code;
     };
     if (cudaSetDevice(b->device) != cudaSuccess) return bail(bfail(b, DNSLBM_ERR_CUDA, "cannot select device"));
+    b->maps_k.assign(n, 0);
     // default launch shape: stages sized for two blocks per SM, the widest
     // consumer set any channel would use alone
     int consumers = 32;
-    for (auto *c : b->ch) consumers = std::max(consumers, c->tma_threads - 32);
-    if (batch_configure(b, kBatchBudget2, 2, consumers) && batch_configure(b, kBatchBudget1, 2, consumers))
+    for (auto *c : b->ch) consumers = std::max(consumers, c->tma_threads - 64);
+    if (batch_configure(b, kBatchBudget1, 2, consumers) && batch_configure(b, kBatchBudget2, 2, consumers))
         return bail(bfail(b, DNSLBM_ERR_ARG, "batched kernel does not fit the device"));
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess ||
@@ -2054,8 +2363,9 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
         cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->fj[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->fj[1], cudaEventDisableTiming) != cudaSuccess ||
-        cudaMalloc(&b->d_counters, sizeof(unsigned) * b->graph_steps) != cudaSuccess ||
-        cudaMalloc(&b->d_arrivals, sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&b->d_flow, sizeof(ChannelLaunch) * 2 * n) != cudaSuccess ||
+        cudaMalloc(&b->d_counter, sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&b->d_maps, sizeof(FlowMaps) * n) != cudaSuccess ||
         cudaMalloc(&b->d_abort, sizeof(int)) != cudaSuccess || cudaMemset(b->d_abort, 0, sizeof(int)) != cudaSuccess)
         return bail(bfail(b, DNSLBM_ERR_CUDA, "batch set-up failed: %s", cudaGetErrorString(cudaGetLastError())));
     *out = b;
@@ -2096,45 +2406,74 @@ static int batch_launch(dnslbm_batch *b, bool odd)
     return DNSLBM_OK;
 }
 
-// The persistent kernel's chunk of n steps from parity `odd`: counters and
-// barrier arrivals cleared, then one cooperative launch.
-static int persist_launch(dnslbm_batch *b, int n, int odd)
+// One launch of the persistent kernel over n steps, with launch table `slot`.
+static int persist_launch(dnslbm_batch *b, int n, int slot)
 {
-    PersistArgs a;
-    a.chans = b->d_launch;
-    a.items = b->d_items;
-    a.nitems = (int)b->items.size();
+    PersistArgs a{};
+    a.chans = b->d_flow + (size_t)slot * b->ch.size();
+    a.maps = b->d_maps;
+    a.nchan = (int)b->ch.size();
     a.nsteps = n;
-    a.first_odd = odd;
     a.stages = b->stages;
     a.stage_bytes = (unsigned)b->pstage;
-    a.counters = b->d_counters;
-    a.arrivals = b->d_arrivals;
+    a.counter = b->d_counter;
     a.abort = b->d_abort;
     a.wait_ns = b->withhold ? b->withhold_wait_ns : b->ch[0]->wait_ns;
     a.withhold = b->withhold;
-    BCK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned) * n, b->stream));
-    BCK(cudaMemsetAsync(b->d_arrivals, 0, sizeof(unsigned), b->stream));
-    BCK(launch_persist_batch(b->precision, a, b->pgrid, b->threads, b->psmem, b->any_q != 0, b->stream));
+    a.eager = 1;
+    BCK(launch_persist_of(b->precision, true, a, b->groups, b->pgrid, b->threads, b->psmem, b->any_q != 0,
+                             b->any_links != 0, b->stream));
+    return DNSLBM_OK;
+}
+
+// The launch table of n steps: the channels one after another, each through
+// all n steps (a small one stays in L2), the blocks moving on to the next
+// channel as they run out of items.
+static int persist_table(dnslbm_batch *b, int n, int slot)
+{
+    std::vector<ChannelLaunch> h(b->ch.size());
+    unsigned first = 0;
+    b->groups = 0;
+    for (size_t i = 0; i < b->ch.size(); ++i) {
+        dnslbm_ctx *c = b->ch[i];
+        if (int rc = flow_reserve(c)) return bfail(b, rc, "channel %zu: %s", i, c->err);
+        flow_maps(c);
+        if (b->maps_k[i] != c->maps_k) {
+            b->maps_k[i] = c->maps_k;
+            BCK(cudaMemcpyAsync(b->d_maps + i, &c->maps, sizeof(FlowMaps), cudaMemcpyHostToDevice, b->stream));
+        }
+        flow_entry(c, flow_order(c, b->pgrid), n, first, h[i]);
+        first = h[i].item_end;
+        b->groups += h[i].flow_groups;
+    }
+    std::vector<ChannelLaunch> &old = b->flow_host[slot];
+    if (old.size() == h.size() && !memcmp((void *)old.data(), (void *)h.data(), sizeof(ChannelLaunch) * h.size()))
+        return DNSLBM_OK;
+    old = h;
+    BCK(cudaMemcpyAsync(b->d_flow + (size_t)slot * h.size(), old.data(), sizeof(ChannelLaunch) * h.size(),
+                        cudaMemcpyHostToDevice, b->stream));
     return DNSLBM_OK;
 }
 
 static int persist_run(dnslbm_batch *b, long nsteps)
 {
-    int odd = b->ch[0]->odd;
     long left = nsteps;
     BCK(cudaMemsetAsync(b->d_abort, 0, sizeof(int), b->stream));
+    double groups = 0;
+    for (auto *c : b->ch) groups += (double)c->tma.gpp * c->nz;
+    const int chunk = std::min(b->graph_steps, flow_chunk(groups));
     while (left > 0) {
-        const int n = (int)std::min<long>(left, b->graph_steps);
-        if (n == b->graph_steps && b->graph_ok && !b->withhold) {
-            cudaGraphExec_t &g = b->graph[odd];
+        const int n = (int)std::min<long>(left, chunk), slot = n == chunk ? 0 : 1;
+        if (int rc = persist_table(b, n, slot)) return rc;
+        if (slot == 0 && b->graph_ok && !b->withhold) {
+            cudaGraphExec_t &g = b->graph[0];
             if (!g) {
                 // the time loop's chunk captured as a graph; a driver that
-                // refuses to capture the cooperative launch leaves plain
-                // launches (noted in the kernel description)
+                // refuses to capture the launch leaves plain launches (noted
+                // in the kernel description)
                 cudaGraph_t graph = nullptr;
                 BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-                const int rc = persist_launch(b, n, odd);
+                const int rc = persist_launch(b, n, slot);
                 cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
                 if (rc == DNSLBM_OK && ee == cudaSuccess) ee = cudaGraphInstantiate(&g, graph, 0);
                 if (graph) cudaGraphDestroy(graph);
@@ -2149,12 +2488,11 @@ static int persist_run(dnslbm_batch *b, long nsteps)
             }
             BCK(cudaGraphLaunch(g, b->stream));
         } else {
-            const int rc = persist_launch(b, n, odd);
+            const int rc = persist_launch(b, n, slot);
             b->withhold = 0;
             if (rc) return rc;
         }
         left -= n;
-        odd = (odd + n) & 1;
     }
     return DNSLBM_OK;
 }
@@ -2200,25 +2538,6 @@ static int batch_run(dnslbm_batch *b, long nsteps, double *ms)
     if (!hl.empty())
         BCK(cudaMemcpyAsync(b->d_links, hl.data(), sizeof(LinksLaunch) * hl.size(), cudaMemcpyHostToDevice,
                             b->stream));
-    if (b->persistent) {
-        // the item table (a new one invalidates the captured graphs, which
-        // hold its address and length)
-        if (b->items.size() > b->d_items_cap) {
-            if (b->d_items) cudaFree(b->d_items);
-            b->d_items = nullptr;
-            b->d_items_cap = 0;
-            BCK(cudaMalloc(&b->d_items, sizeof(BatchItem) * b->items.size()));
-            b->d_items_cap = b->items.size();
-            destroy_graphs(b);
-        }
-        if (b->items.size() != b->items_uploaded.size() ||
-            memcmp(b->items.data(), b->items_uploaded.data(), sizeof(BatchItem) * b->items.size())) {
-            destroy_graphs(b);
-            b->items_uploaded = b->items;
-        }
-        BCK(cudaMemcpyAsync(b->d_items, b->items.data(), sizeof(BatchItem) * b->items.size(),
-                            cudaMemcpyHostToDevice, b->stream));
-    }
     int odd = b->ch[0]->odd;
     long left = nsteps;
     if (ms) BCK(cudaEventRecord(b->ev[0], b->stream));
@@ -2307,10 +2626,9 @@ extern "C" const char *dnslbm_batch_kernel(const dnslbm_batch *b)
     if (!b) return "";
     if (b->persistent) {
         snprintf(buf, sizeof buf,
-                 "persist_batch_kernel<fp%d>: %zu channels, %zu items per step, %d blocks x %d threads, %d stages, "
-                 "%zu B smem; one cooperative launch per %d steps, CUDA graph%s",
-                 b->precision, b->ch.size(), b->items.size(), b->pgrid, b->threads, b->stages, b->psmem,
-                 b->graph_steps, b->graph_note);
+                 "persist_batch_kernel<fp%d>: %zu channels, %d blocks x %d threads, %d stages, %zu B smem; one launch "
+                 "per %d steps, CUDA graph%s",
+                 b->precision, b->ch.size(), b->pgrid, b->threads, b->stages, b->psmem, b->graph_steps, b->graph_note);
         return buf;
     }
     snprintf(buf, sizeof buf, "step_tma_batch_kernel<fp%d>: %zu channels, %d blocks x %d threads, %d stages, %zu B smem"
@@ -2330,7 +2648,7 @@ extern "C" int dnslbm_batch_autotune(dnslbm_batch *b, int steps, char *report, s
     if (steps >= b->graph_steps) steps = b->graph_steps - 1;  // plain launches, no graph to capture
     BCK(cudaSetDevice(b->device));
     size_t bb = b->budget;
-    int bs = b->stages, bc = b->threads - 32, ncand = 0;
+    int bs = b->stages, bc = b->threads - (b->persistent ? 64 : 32), ncand = 0;
     double best = 1e30;
     for (size_t budget : {kBatchBudget1, kBatchBudget2, kBatchBudget3})
         for (int st : {2, 3, 4})
@@ -2344,22 +2662,6 @@ extern "C" int dnslbm_batch_autotune(dnslbm_batch *b, int steps, char *report, s
                 ++ncand;
                 if (ms < best) best = ms, bb = budget, bs = st, bc = cons;
             }
-    // the persistent kernel: how finely each step's work is cut, at the best shape
-    if (b->persistent) {
-        int bi = b->items_per_block;
-        for (int ipb : {2, 8, 16}) {
-            b->items_per_block = ipb;
-            if (batch_configure(b, bb, bs, bc)) continue;
-            int rc = DNSLBM_OK;
-            for (auto *c : b->ch)
-                if ((rc = dnslbm_init_rest(c))) return bfail(b, rc, "%s", c->err);
-            double ms = 0;
-            if ((rc = batch_run(b, 2, nullptr)) || (rc = batch_run(b, steps, &ms))) return rc;
-            ++ncand;
-            if (ms < best) best = ms, bi = ipb;
-        }
-        b->items_per_block = bi;
-    }
     // leave the channels as created: no state, counters clear
     for (auto *c : b->ch) {
         int rc = reset_counters(c);

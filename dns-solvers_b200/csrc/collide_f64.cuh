@@ -46,6 +46,29 @@ struct F64Cell {
     double dens, jx, u0, u1, u2;
 };
 
+// Population A and its opposite B after the collision.  Rounding is symmetric
+// in sign, so e_B . u == -(e_A . u) exactly and the pair shares the products
+// of e . u: 3 (e.u), 4.5 (e.u)^2 and 9 (e.u) are computed once.
+template <int A>
+__device__ __forceinline__ void f64_pair(double (&f)[Q], const F64Cell &c, double v15, const double (&wd)[3], double m3,
+                                         double p3, double n3, double omega, double G)
+{
+    constexpr int B = lat_opp(A), ex = lat_ex(A), cls = lat_wclass(A);
+    constexpr double w = cls == 1 ? 1. / 18. : 1. / 36.;
+    const double u = f64_eu<A>(c.u0, c.u1, c.u2);
+    const double u3 = 3. * u, uu = (4.5 * u) * u;
+    const double ta = ((1. + u3) + uu) - v15, tb = ((1. - u3) + uu) - v15;
+    double bra = m3, brb = m3;
+    if (ex != 0) {
+        const double u9 = 9. * u;
+        bra = ex > 0 ? p3 + u9 : n3 - u9;
+        brb = ex > 0 ? n3 + u9 : p3 - u9;
+    }
+    const double Fa = (w * bra) * G, Fb = ex != 0 ? (w * brb) * G : Fa;
+    f[A] = f[A] + (Fa - omega * (f[A] - wd[cls] * ta));
+    f[B] = f[B] + (Fb - omega * (f[B] - wd[cls] * tb));
+}
+
 // BGK collision with the reference's forcing term, in place.
 __device__ __forceinline__ F64Cell f64_collide(double (&f)[Q], double omega, double G)
 {
@@ -57,23 +80,13 @@ __device__ __forceinline__ F64Cell f64_collide(double (&f)[Q], double omega, dou
     c.u2 = jz / c.dens;
     const double v15 = 1.5 * (c.u0 * c.u0 + c.u1 * c.u1 + c.u2 * c.u2);
     const double wd[3] = {(1. / 3.) * c.dens, (1. / 18.) * c.dens, (1. / 36.) * c.dens};
-    const double wc[3] = {1. / 3., 1. / 18., 1. / 36.};
     const double m3 = 3. * (0. - c.u0), p3 = 3. * (1. - c.u0), n3 = 3. * (-1. - c.u0);
-#pragma unroll
-    for (int a = 0; a < Q; ++a) {
-        double u;
-        switch (a) {  // unrolled: one case survives per a
-#define EU(A) case A: u = f64_eu<A>(c.u0, c.u1, c.u2); break;
-            EU(0) EU(1) EU(2) EU(3) EU(4) EU(5) EU(6) EU(7) EU(8) EU(9)
-            EU(10) EU(11) EU(12) EU(13) EU(14) EU(15) EU(16) EU(17) EU(18)
-#undef EU
-        }
-        const double t = ((1. + 3. * u) + (4.5 * u) * u) - v15;
-        const double feq = wd[lat_wclass(a)] * t;
-        const double br = lat_ex(a) == 0 ? m3 : lat_ex(a) > 0 ? p3 + 9. * u : n3 - 9. * u;
-        const double Fi = (wc[lat_wclass(a)] * br) * G;
-        f[a] = f[a] + (Fi - omega * (f[a] - feq));
-    }
+    // rest direction: e . u = 0
+    f[0] = f[0] + (((1. / 3.) * m3) * G - omega * (f[0] - wd[0] * (1. - v15)));
+#define DNSLBM_PAIR(A) f64_pair<A>(f, c, v15, wd, m3, p3, n3, omega, G);
+    DNSLBM_PAIR(1) DNSLBM_PAIR(3) DNSLBM_PAIR(5) DNSLBM_PAIR(7) DNSLBM_PAIR(8) DNSLBM_PAIR(11) DNSLBM_PAIR(12)
+    DNSLBM_PAIR(15) DNSLBM_PAIR(16)
+#undef DNSLBM_PAIR
     return c;
 }
 

@@ -66,6 +66,17 @@ __host__ __device__ __forceinline__ constexpr int wall_link(int a)
     return lat_ex(a) == 1 ? 1 : lat_ex(a) == -1 ? 2 : lat_ey(a) == 1 ? 3 : lat_ey(a) == -1 ? 4 : 0;
 }
 
+// Order of the population arrays in device memory, and of the directions'
+// rows in a shared-memory stage: directions with the same (e_y, e_z), whose
+// rows of an odd step lie side by side, follow one another, so one tensor
+// copy moves the three of a group (positions 0-2, 3-5, 6-8, 9-11, 12-14; the
+// last four directions have a row position each).
+__host__ __device__ __forceinline__ constexpr int lat_pos(int a)
+{
+    return a <= 1 ? a : a == 2 ? 2 : a == 3 ? 3 : a == 7 ? 4 : a == 8 ? 5 : a == 4 ? 6 : a == 9 ? 7 : a == 10 ? 8
+         : a == 5 ? 9 : a == 11 ? 10 : a == 14 ? 11 : a == 6 ? 12 : a == 12 ? 13 : a == 13 ? 14 : a;
+}
+
 struct Dims {
     int nx, ny, nz;  // fluid cells
 };

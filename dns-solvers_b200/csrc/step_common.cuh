@@ -29,7 +29,7 @@ struct StepArgs {
     double omega, ubulk, gx;
     int const_q;
     double *force;           // [2] force of step s is force[s & 1]
-    double *shift;           // [2][nz][3] plane means of the previous state
+    double *shift;           // plane means of an earlier state, see shift_entry
     long long *step_ctr;     // steps done (advanced by the step tail)
     double *partials;        // [nz][slots][NP]
     double *plane_sums;      // [nz][NP]
@@ -42,6 +42,7 @@ struct StepArgs {
     // plane of a solid cell carry a per-cell link mask, see cell_links
     const int *band_of;      // [nz] index of the plane's mask block, -1: none
     const unsigned *links;   // [nband][ny][nx]
+    const unsigned long long *link_rows;  // [nband][ny] the rows of those planes, see RowInfo
     // bounded waits of the row-pipelined kernels: a wait gives up after
     // wait_ns of the GPU's global timer (status[1] set); withhold_stage is a
     // test switch (0 otherwise) that makes one block withhold a load
@@ -54,7 +55,20 @@ struct StepArgs {
     // the step tail (whole channels: 1, 1, 1)
     int wall_lo = 1, wall_hi = 1;
     int tail = 1;
+    // entries of the shift array: 0 for [2][nz][3] (step s reads the means
+    // of the state before it), else a power of two R for [R][nz][3] (step s
+    // reads the means of state s - R, or of the loaded state)
+    int ring = 0;
 };
+
+// The shift c(z) of a step's energy sum: the plane means entry it reads.
+// Any recent means serve (the shift only keeps the one-pass variance free of
+// cancellation).  A ring lets steps overlap: step s needs no sums of the
+// steps just before it.
+__device__ __forceinline__ const double *shift_entry(const StepArgs &p, long long step)
+{
+    return p.shift + (size_t)(step & (p.ring ? p.ring - 1 : 1)) * p.nz * 3;
+}
 
 // -1: plane z lies next to the bottom wall, +1: next to the top wall, 0:
 // between fluid planes (a ghost plane of a slab included)
@@ -89,6 +103,23 @@ __device__ __forceinline__ unsigned cell_links(const int *band_of, const unsigne
     const int b = band_of[z];
     return b < 0 ? 0u : links[((size_t)b * ny + y) * nx + x];
 }
+
+// A row of a plane with link masks whose cells are alike (streamwise riblets:
+// every row): bit 63 set, bit 62 for a row of solid cells, and per direction
+// A two bits at 2 A: 0 streams, 1 bounces back, 2 reflects specularly.  Then
+// each direction of the row is one whole population row, in an odd step too,
+// which no other row touches.  0: a mixed row.
+struct RowInfo {
+    static constexpr unsigned long long kAlike = 1ull << 63, kSolid = 1ull << 62;
+    static __host__ __device__ __forceinline__ int link(unsigned long long r, int a) { return (int)(r >> (2 * a)) & 3; }
+    // the link mask of the row's cells
+    static __host__ __device__ __forceinline__ unsigned mask(unsigned long long r)
+    {
+        unsigned m = (r & kSolid) ? 1u : 0u;
+        for (int a = 1; a < Q; ++a) m |= link(r, a) == 1 ? 1u << a : 0u;
+        return m;
+    }
+};
 
 // ---------------------------------------------------------------- addresses
 // Neighbourhood of a cell: wrapped x and the 9 row offsets (dy, dz).
@@ -224,17 +255,18 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *smem)
 //         the current step from the reader-side totals, nothing logged).
 // step < 0 (mode 0): the step is read from the step counter (the tail is
 // its only writer, once per step).
-static __device__ __forceinline__ void step_tail(const StepArgs &a, long long step, double force_used, int mode, double *smem,
-                                                 int nthreads)
+// Two parts, shared by the block-wide tail below and the persistent
+// kernel's one-warp tail: the sums over the planes (this thread's planes z0,
+// z0 + stride, ...), and the record of the summed totals.
+__device__ __forceinline__ void tail_planes(const StepArgs &a, long long step, int mode, const double *plane_sums, int z0,
+                                            int stride, double (&t)[6])
 {
-    if (step < 0) step = __ldcg(a.step_ctr);
     const int nz = a.nz;
     const double np = (double)a.nx * (double)a.ny;
-    const double *cshift = a.shift + (size_t)(step & 1) * nz * 3;
-    double *nshift = a.shift + (size_t)((mode == 0 ? step + 1 : step) & 1) * nz * 3;
-    double t[6] = {0, 0, 0, 0, 0, 0};  // rho, jx, sum of plane means u, K, writer rho, writer jx
-    for (int z = threadIdx.x; z < nz; z += nthreads) {
-        const double *ps = a.plane_sums + (size_t)z * NP;
+    const double *cshift = shift_entry(a, step);
+    double *nshift = const_cast<double *>(a.ring || mode != 0 ? shift_entry(a, step) : shift_entry(a, step + 1));
+    for (int z = z0; z < nz; z += stride) {
+        const double *ps = plane_sums + (size_t)z * NP;
         double s[NP];
 #pragma unroll
         for (int i = 0; i < NP; ++i) s[i] = __ldcg(ps + i);
@@ -247,12 +279,22 @@ static __device__ __forceinline__ void step_tail(const StepArgs &a, long long st
         t[3] += 0.5 * (s[5] - np * (du * du + dv * dv + dw * dw));
         t[4] += s[6];
         t[5] += s[7];
-        nshift[z * 3 + 0] = um;
-        nshift[z * 3 + 1] = vm;
-        nshift[z * 3 + 2] = wm;
+        // a loaded state fills every entry of a ring
+        const int copies = a.ring && mode != 0 ? a.ring : 1;
+        for (int r = 0; r < copies; ++r) {
+            double *n = copies > 1 ? a.shift + (size_t)r * nz * 3 : nshift;
+            n[z * 3 + 0] = um;
+            n[z * 3 + 1] = vm;
+            n[z * 3 + 2] = wm;
+        }
     }
-    block_sum<6>(t, smem, nthreads);
-    if (threadIdx.x != 0) return;
+}
+
+__device__ __forceinline__ void tail_record(const StepArgs &a, long long step, double force_used, int mode,
+                                            const double *plane_sums, const double (&t)[6])
+{
+    const int nz = a.nz;
+    const double np = (double)a.nx * (double)a.ny;
     const double N = np * (double)nz;
     const double rho = t[0] / N, momentum = t[1] / N;
     if (mode == 1) {
@@ -260,10 +302,10 @@ static __device__ __forceinline__ void step_tail(const StepArgs &a, long long st
         return;
     }
     // wall shear stress, wshearstr.c:24-121 (top density from plane zd-4)
-    auto umean = [&](int z) { return __ldcg(a.plane_sums + (size_t)z * NP + 2) / np; };
+    auto umean = [&](int z) { return __ldcg(plane_sums + (size_t)z * NP + 2) / np; };
     const double mu = (1. / 6.) * (2. / a.omega - 1);
-    const double davg_dn = __ldcg(a.plane_sums + 0 * NP + 0) / np;
-    const double davg_up = __ldcg(a.plane_sums + (size_t)(nz - 3) * NP + 0) / np;
+    const double davg_dn = __ldcg(plane_sums + 0 * NP + 0) / np;
+    const double davg_up = __ldcg(plane_sums + (size_t)(nz - 3) * NP + 0) / np;
     double stdown = -2. * umean(0) + 3. * umean(1) - umean(2);
     double stup = -(2. * umean(nz - 1) - 3. * umean(nz - 2) + umean(nz - 3));
     stdown *= mu * davg_dn;
@@ -283,7 +325,18 @@ static __device__ __forceinline__ void step_tail(const StepArgs &a, long long st
     // constant-Q: next force from the totals of the state this step wrote
     // (encalc.c:121 evaluated one step ahead); sum of populations = t[4]
     a.force[(step + 1) & 1] = a.const_q ? (t[4] / N) * a.ubulk - t[5] / N : a.gx;
-    *a.step_ctr = step + 1;
+}
+
+static __device__ __forceinline__ void step_tail(const StepArgs &a, long long step, double force_used, int mode, double *smem,
+                                                 int nthreads)
+{
+    if (step < 0) step = __ldcg(a.step_ctr);
+    double t[6] = {0, 0, 0, 0, 0, 0};  // rho, jx, sum of plane means u, K, writer rho, writer jx
+    tail_planes(a, step, mode, a.plane_sums, threadIdx.x, nthreads, t);
+    block_sum<6>(t, smem, nthreads);
+    if (threadIdx.x != 0) return;
+    tail_record(a, step, force_used, mode, a.plane_sums, t);
+    if (mode == 0) *a.step_ctr = step + 1;
 }
 
 // One block's contribution to plane z: block partials -> (last contributor

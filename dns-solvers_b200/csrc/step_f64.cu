@@ -29,9 +29,9 @@ __global__ void __launch_bounds__(128, 4) step_f64_kernel(const StepArgs p)
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int z = blockIdx.z;
     const int wall = plane_wall(p, z);
-    const double c0 = p.shift[(size_t)(step & 1) * p.nz * 3 + z * 3 + 0];
-    const double c1 = p.shift[(size_t)(step & 1) * p.nz * 3 + z * 3 + 1];
-    const double c2 = p.shift[(size_t)(step & 1) * p.nz * 3 + z * 3 + 2];
+    const double c0 = shift_entry(p, step)[z * 3 + 0];
+    const double c1 = shift_entry(p, step)[z * 3 + 1];
+    const double c2 = shift_entry(p, step)[z * 3 + 2];
     double acc[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) acc[i] = 0.0;

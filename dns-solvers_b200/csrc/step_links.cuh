@@ -20,6 +20,17 @@
 
 namespace dnslbm {
 
+// Place of direction a's rows in a shared-memory stage: the order of the
+// population arrays (lat_pos) in the persistent kernel, whose tensor copies
+// need it; the lattice's order in the kernels of one launch per step, whose
+// row copies land slower in the other (1256x157x100 FP64 1216 against 1126
+// us/step).
+#ifdef DNSLBM_GROUPED_STAGE
+__host__ __device__ __forceinline__ constexpr int stage_pos(int a) { return lat_pos(a); }
+#else
+__host__ __device__ __forceinline__ constexpr int stage_pos(int a) { return a; }
+#endif
+
 template <typename T>
 using RegT = typename std::conditional<std::is_same<T, double>::value, double, float>::type;
 
@@ -131,26 +142,29 @@ __device__ __forceinline__ void solid_sums(const RegT<T> (&f)[Q], double c0, dou
 
 // One cell with link mask `lk` (plane `wall` = -1 bottom, +1 top, 0
 // interior).  Even step: the cell's own populations, from shared memory at
-// sbx[A * dstride] when sbx is given (the bulk-copied own rows), else from
+// sbx[stage_pos(A) * dstride] when sbx is given (the bulk-copied own rows), else from
 // global memory.  Odd step: global memory through the link addresses, except
 // that with sbx given (the bulk-copied rows of the odd address set, element
 // x at sbx, x - 1 at sbx + om, x + 1 at sbx + op) a link that neither
 // bounces nor meets a wall is read from shared memory; the odd step's
-// results always go to global memory.
+// results always go to global memory.  `alike`: a row of cells alike
+// (RowInfo), whose 19 rows are all at sbx (the shifted ones as above, a
+// bounced link's at the cell's own column) and take the results.
 // FP64 sums go to acc; low-precision sums go to racc (FP32, flushed by the
 // caller) except the cell counts, which go to acc[0] and acc[6].
 template <typename T, bool ODD, bool CONSTQ>
 __device__ __forceinline__ void links_cell(const StepArgs &p, const Nbr &n, int wall, unsigned lk, T *sbx, int dstride,
                                            double G, double c0, double c1, double c2, double (&acc)[NP],
-                                           float (&racc)[NP], int om = 0, int op = 0)
+                                           float (&racc)[NP], int om = 0, int op = 0, bool alike = false)
 {
     using V = RegT<T>;
+    if (!ODD) alike = false;
     if (lk & 1u) {
         // a solid cell holds the (symmetric) rest state in its own slots
         V f[Q];
 #pragma unroll
         for (int A = 0; A < Q; ++A)
-            f[A] = (!ODD && sbx) ? ld_raw<T>(sbx + A * dstride) : ld_glb<T>(static_cast<const T *>(p.pop[A]) + n.c0);
+            f[A] = (sbx && (!ODD || alike)) ? ld_raw<T>(sbx + stage_pos(A) * dstride) : ld_glb<T>(static_cast<const T *>(p.pop[A]) + n.c0);
         solid_sums<T, CONSTQ>(f, c0, c1, c2, acc, racc);
         return;
     }
@@ -159,10 +173,10 @@ __device__ __forceinline__ void links_cell(const StepArgs &p, const Nbr &n, int 
         constexpr int A = decltype(ac)::value;
         V v;
         constexpr int ex = lat_ex(A), ez = lat_ez(A);
-        if (!ODD && sbx) v = ld_raw<T>(sbx + A * dstride);
+        if (!ODD && sbx) v = ld_raw<T>(sbx + stage_pos(A) * dstride);
         else if (!ODD) v = ld_glb<T>(static_cast<const T *>(p.pop[A]) + n.c0);
-        else if (sbx && !((lk >> A) & 1u) && !(ez != 0 && wall == ez))
-            v = ld_raw<T>(sbx + A * dstride + (ex > 0 ? op : (ex < 0 ? om : 0)));
+        else if (alike || (sbx && !((lk >> A) & 1u) && !(ez != 0 && wall == ez)))
+            v = ld_raw<T>(sbx + stage_pos(A) * dstride + (((lk >> A) & 1u) ? 0 : (ex > 0 ? op : (ex < 0 ? om : 0))));
         else v = ld_glb<T>(links_ptr<T, A>(p, n, wall, lk));
         f[ODD ? lat_opp(A) : A] = v;
     });
@@ -225,7 +239,9 @@ __device__ __forceinline__ void links_cell(const StepArgs &p, const Nbr &n, int 
     static_for<Q>([&](auto ac) {
         constexpr int A = decltype(ac)::value;
         const V v = f[ODD ? A : lat_opp(A)];
-        if (!ODD && sbx) st_raw<T>(sbx + A * dstride, v);
+        constexpr int ex = lat_ex(A);
+        if (!ODD && sbx) st_raw<T>(sbx + stage_pos(A) * dstride, v);
+        else if (alike) st_raw<T>(sbx + stage_pos(A) * dstride + (((lk >> A) & 1u) ? 0 : (ex > 0 ? op : (ex < 0 ? om : 0))), v);
         else if (!ODD) st_raw<T>(static_cast<T *>(p.pop[A]) + n.c0, v);
         else st_raw<T>(links_ptr<T, A>(p, n, wall, lk), v);
     });
@@ -256,7 +272,7 @@ __device__ __forceinline__ void links_pass_body(const LinksLaunch &L, int blk)
     const int wall = plane_wall(p, z);
     const long long step = *p.step_ctr;
     const double G = CONSTQ ? p.force[step & 1] : p.gx;
-    const double *sh = p.shift + (size_t)(step & 1) * p.nz * 3 + z * 3;
+    const double *sh = shift_entry(p, step) + z * 3;
     const double c0 = sh[0], c1 = sh[1], c2 = sh[2];
     double acc[NP];
 #pragma unroll

@@ -230,7 +230,7 @@ __device__ __forceinline__ void copy_segment(const StepArgs &p, const GroupRows 
 
 // ------------------------------------------------------------------ cells
 // The k cell rows of a row group from the stage buffer: direction A's
-// element x of row j at sb[A * dstride + j * pitch + x].  The group's k * nx
+// element x of row j at sb[stage_pos(A) * dstride + j * pitch + x].  The group's k * nx
 // cells are spread over the nc consumer threads as one range, so rows
 // shorter than the consumer set keep every thread busy.
 // WALL: 0 interior plane, -1 bottom plane, +1 top plane.
@@ -287,7 +287,7 @@ __device__ __forceinline__ void tma_group(const StepArgs &p, T *sb, int dstride,
             } else {
                 const int xs = (ODD && !wdir) ? (lat_ex(A) > 0 ? xp : (lat_ex(A) < 0 ? xm : x)) : x;
                 if (SEG && edge && !wdir && lat_ex(A) != 0) v = ld_glb<T>(shifted_ptr(A, xs));
-                else v = ld_raw<T>(sbj + A * dstride + xs);
+                else v = ld_raw<T>(sbj + stage_pos(A) * dstride + xs);
             }
             f[ODD ? lat_opp(A) : A] = v;
         }
@@ -363,9 +363,9 @@ __device__ __forceinline__ void tma_group(const StepArgs &p, T *sb, int dstride,
                 const int xs = (ODD && !wdir) ? (lat_ex(A) > 0 ? xp : (lat_ex(A) < 0 ? xm : x)) : x;
                 if (SEG && edge && !wdir && lat_ex(A) != 0) {
                     st_raw<T>(shifted_ptr(A, xs), v);
-                    if ((unsigned)(xs + sxoff) < (unsigned)dstride) st_raw<T>(sbj + A * dstride + xs, v);
+                    if ((unsigned)(xs + sxoff) < (unsigned)dstride) st_raw<T>(sbj + stage_pos(A) * dstride + xs, v);
                 } else {
-                    st_raw<T>(sbj + A * dstride + xs, v);
+                    st_raw<T>(sbj + stage_pos(A) * dstride + xs, v);
                 }
             }
         }
@@ -454,7 +454,7 @@ __device__ __forceinline__ void tma_group2(const StepArgs &p, const LpParams &lk
 #pragma unroll
         for (int A = 0; A < Q; ++A) {
             const bool wdir = ODD && lat_ez(A) != 0 && lat_ez(A) == WALL;
-            const T *row = sbj + A * dstride;
+            const T *row = sbj + stage_pos(A) * dstride;
             float2 v;
             if (!ODD || wdir || lat_ex(A) == 0) v = IO::ld2(row + x);
             else if (lat_ex(A) > 0) v = make_float2(IO::ld1(row + xp0), IO::ld1(row + xp1));
@@ -467,7 +467,7 @@ __device__ __forceinline__ void tma_group2(const StepArgs &p, const LpParams &lk
         auto emit = [&](int a) {
             const int A = ODD ? a : lat_opp(a);
             const bool wdir = ODD && lat_ez(A) != 0 && lat_ez(A) == WALL;
-            T *row = sbj + A * dstride;
+            T *row = sbj + stage_pos(A) * dstride;
             const float2 v = f[a];
             if (!ODD || wdir || lat_ex(A) == 0) {
                 IO::st2(row + x, v);  // for a one-cell pair the second lane lands in the row padding
@@ -585,9 +585,9 @@ __device__ __forceinline__ void tma_producer(const StepArgs &p, const TmaArgs &t
                     if (t.nseg > 1) {
                         int x0, x1;
                         group_xrange(t, gi, p.nx, x0, x1);
-                        copy_segment<T>(p, g, x0, x1, shift_of(wall), stage + (size_t)lane * dir_bytes, false, nullptr);
+                        copy_segment<T>(p, g, x0, x1, shift_of(wall), stage + (size_t)stage_pos(lane) * dir_bytes, false, nullptr);
                     } else {
-                        copy_group<T>(p, t, g, k, stage + (size_t)lane * dir_bytes, false, nullptr);
+                        copy_group<T>(p, t, g, k, stage + (size_t)stage_pos(lane) * dir_bytes, false, nullptr);
                     }
                 }
                 bulk_commit();
@@ -614,9 +614,9 @@ __device__ __forceinline__ void tma_producer(const StepArgs &p, const TmaArgs &t
                 __syncwarp();
                 if (lane < Q && g.bulk) {
                     if (t.nseg > 1)
-                        copy_segment<T>(p, g, x0, x1, shift_of(wall), stage + (size_t)lane * dir_bytes, true, full + st);
+                        copy_segment<T>(p, g, x0, x1, shift_of(wall), stage + (size_t)stage_pos(lane) * dir_bytes, true, full + st);
                     else
-                        copy_group<T>(p, t, g, k, stage + (size_t)lane * dir_bytes, true, full + st);
+                        copy_group<T>(p, t, g, k, stage + (size_t)stage_pos(lane) * dir_bytes, true, full + st);
                 }
                 loaded |= 1u << st;
                 phase = (phase & ~(1u << st)) | ((unsigned)((i / S) & 1) << st);
@@ -711,7 +711,7 @@ __device__ __forceinline__ void tma_step_body(const StepArgs &p, const TmaArgs &
 
     const long long step = *p.step_ctr;
     const double G = CONSTQ ? p.force[step & 1] : p.gx;
-    const double *shift_now = p.shift + (size_t)(step & 1) * p.nz * 3;
+    const double *shift_now = shift_entry(p, step);
     const int dstride = t.dir_elems;
     [[maybe_unused]] const LpParams lk = lp_params<typename std::conditional<std::is_same<T, double>::value, float, T>::type>(
         (float)p.omega, (float)G);
@@ -791,6 +791,19 @@ struct ChannelLaunch {
     TmaArgs t;
     int first_block;
     int textured;  // TEX of the channel (0 smooth, else textured walls)
+    // the persistent kernel (step_persist.cuh): the channel's items are the
+    // positions [item_first, item_end) of the launch's sequence
+    unsigned item_first, item_end;
+    int depth, lag;        // steps run at once, distance between them in row groups
+    unsigned flow_groups;  // row groups of all planes (nz * gpp)
+    size_t pop_bytes;      // bytes between two population arrays
+    int tensor;            // the channel's tensor maps are valid
+    unsigned *flags;       // [flow_groups] steps of the launch a group is done with
+    long long *base;       // step counter at the start of the launch
+    double *fpart;         // [ring][nz][gpp][NP] sums of the row groups
+    double *fsums;         // [ring][nz][NP] plane sums
+    unsigned *fctr;        // [ring][nz] groups of the plane done
+    unsigned *ftotal;      // [ring] planes of the step done
 };
 
 template <typename T, bool ODD>
