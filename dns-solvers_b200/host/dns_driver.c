@@ -386,6 +386,9 @@ int main(int argc, char **argv)
     while (ss < up + 1 && !nan_stop) {
         if (!(ss % utime)) {
             Snapshot *sn = &snap[nout & 1];
+            /* the writer may still be at this set's event before last: its
+             * label names the files */
+            if (D.ASYNC && nout > 1 && writer_wait(&W)) return die(c, DNSLBM_ERR_IO, "writing an output file");
             sn->label = TM + ss / utime;
             sn->checkpoint = !(ss % (10 * utime));
             if (sn->checkpoint && (rc = dnslbm_get_force(c, &sn->force))) return die(c, rc, "dnslbm_get_force");
