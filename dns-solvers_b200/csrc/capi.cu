@@ -25,13 +25,14 @@ void launch_stats(int precision, const IoArgs &p, dim3 grid, dim3 block, int row
 void launch_stats_sample(int nz, double np, const double *planes, double *mean, double *acc, bool accumulate,
                          cudaStream_t s);
 void launch_stats_rows(int nz, double np, const double *mean, const double *planes, double *out, cudaStream_t s);
-void launch_quadrant(const double *vel, int nx, int ny, int zd, double *mean, double *out, cudaStream_t s);
-size_t correlation_scratch(int nx, int ny, int zd, int per_chunk);
+size_t quadrant_scratch(int nx, int ny, int zd);
+void launch_quadrant(const double *vel, int nx, int ny, int zd, double *scratch, double *mean, double *out, cudaStream_t s);
+size_t correlation_scratch(int nx, int ny, int zd);
 int correlation_max_line();
-cudaError_t launch_correlations(const double *vel, int nx, int ny, int zd, int per_chunk, double *scratch,
-                                double *xcorl, double *ycorl, double *ua, cudaStream_t s);
-size_t spectra_scratch(int nx, int ny, int zd, int jb);
-cudaError_t launch_spectra(const double *vel, int nx, int ny, int zd, int jb, double *scratch, double *ex, double *ey,
+cudaError_t launch_correlations(const double *vel, int nx, int ny, int zd, double *scratch, double *xcorl, double *ycorl,
+                                double *ua, cudaStream_t s);
+size_t spectra_scratch(int nx, int ny, int zd);
+cudaError_t launch_spectra(const double *vel, int nx, int ny, int zd, double *scratch, double *ex, double *ey,
                            cudaStream_t s);
 #define DNSLBM_PERSIST_DECL(S)                                                                                      \
     int persist_prepare_##S(int threads, size_t smem, bool any_q, bool links);                                                                          \
@@ -152,6 +153,8 @@ struct dnslbm_ctx {
     cudaEvent_t out_ev[2] = {nullptr, nullptr};
     int out_pending = 0;
     double *quad_buf = nullptr;  // quadrant analysis: plane means [zd][3], plane sums [zd][9]
+    double *post_ws = nullptr;   // scratch and results of the post-processing calls, kept between calls
+    size_t post_ws_n = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> tev;  // per-launch timing events
     dim3 grid, block;
@@ -291,7 +294,7 @@ static void free_all(dnslbm_ctx *c)
                     c->band_of,    c->links,      c->plane_list,    c->d_llaunch,   c->stat_acc,
                     c->out_lbf,    c->out_vel,    c->out_den,       c->out_stats,   c->quad_buf,
                     c->shift_all,  c->flow_flags,    c->flow_part,   c->flow_sums,
-                    c->flow_ctr,   c->flow_base,  c->link_rows};
+                    c->flow_ctr,   c->flow_base,  c->link_rows,     c->post_ws};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (auto &e : c->ev)
@@ -1653,6 +1656,23 @@ static void quadrant_finish(int zd, double n, const double *sums, double *quadra
     }
 }
 
+// At least n doubles of the context's post-processing workspace.
+static int post_reserve(dnslbm_ctx *c, size_t n)
+{
+    if (n <= c->post_ws_n) return DNSLBM_OK;
+    if (c->post_ws) CK(cudaFree(c->post_ws));
+    c->post_ws = nullptr;
+    c->post_ws_n = 0;
+    const cudaError_t e = cudaMalloc((void **)&c->post_ws, n * sizeof(double));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes of post-processing workspace failed: %s",
+                    n * sizeof(double), cudaGetErrorString(e));
+    }
+    c->post_ws_n = n;
+    return DNSLBM_OK;
+}
+
 extern "C" int dnslbm_quadrant(dnslbm_ctx *c, double *quadrant, double *dquadrant, double *uw)
 {
     if (!c) return fail(c, DNSLBM_ERR_ARG, "null context");
@@ -1668,7 +1688,8 @@ extern "C" int dnslbm_quadrant(dnslbm_ctx *c, double *quadrant, double *dquadran
     // the velocity field in the vel layout, then the two plane passes
     if (c->out_pending) CK(cudaStreamWaitEvent(c->stream, c->out_ev[1], 0));
     launch_io(c->deck.precision, 3, io_args(c), 0, c->nx, c->out_vel, c->out_den, c->stream);
-    launch_quadrant(c->out_vel, c->nx, c->ny, zd, c->quad_buf, c->quad_buf + (size_t)zd * 3, c->stream);
+    if ((rc = post_reserve(c, quadrant_scratch(c->nx, c->ny, zd)))) return rc;
+    launch_quadrant(c->out_vel, c->nx, c->ny, zd, c->post_ws, c->quad_buf, c->quad_buf + (size_t)zd * 3, c->stream);
     CK(cudaGetLastError());
     std::vector<double> sums((size_t)zd * 9);
     CK(cudaMemcpyAsync(sums.data(), c->quad_buf + (size_t)zd * 3, sums.size() * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1689,11 +1710,11 @@ extern "C" int dnslbm_quadrant_vel(const double *vel, int xdv, int ydv, int zdv,
     CK(cudaSetDevice(device));
     double *dv = nullptr, *buf = nullptr;
     cudaError_t e = cudaMalloc(&dv, n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&buf, (size_t)zd * 12 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&buf, ((size_t)zd * 12 + quadrant_scratch(xdv, ydv, zd)) * sizeof(double));
     std::vector<double> sums((size_t)zd * 9);
     if (e == cudaSuccess) e = cudaMemcpy(dv, vel, n * sizeof(double), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
-        launch_quadrant(dv, xdv, ydv, zd, buf, buf + (size_t)zd * 3, 0);
+        launch_quadrant(dv, xdv, ydv, zd, buf + (size_t)zd * 12, buf, buf + (size_t)zd * 3, 0);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
@@ -1709,28 +1730,30 @@ extern "C" int dnslbm_quadrant_vel(const double *vel, int xdv, int ydv, int zdv,
 // ycorrel.c) of a velocity field already in device memory: temporary device
 // memory for the fluctuations and the partial sums, results copied to the
 // caller's host arrays (any may be NULL).
-constexpr int kCorrLinesPerChunk = 8;
+//
+// ws: a workspace of correlations_ws doubles, or nullptr for a temporary one.
+static size_t correlations_ws(int nx, int ny, int zd) { return correlation_scratch(nx, ny, zd) + (size_t)zd * 3 * (nx + ny + 1); }
 
-static cudaError_t correlations_of(const double *dvel, int nx, int ny, int zd, cudaStream_t s, double *xcorl,
+static cudaError_t correlations_of(const double *dvel, int nx, int ny, int zd, cudaStream_t s, double *ws, double *xcorl,
                                    double *ycorl, double *uavg)
 {
-    double *scratch = nullptr, *res = nullptr;
+    double *own = nullptr;
     const size_t nres = (size_t)zd * 3 * (nx + ny + 1);
-    cudaError_t e = cudaMalloc(&scratch, correlation_scratch(nx, ny, zd, kCorrLinesPerChunk) * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&res, nres * sizeof(double));
-    double *dx = res, *dy = res + (size_t)zd * 3 * nx, *du = dy + (size_t)zd * 3 * ny;
-    if (e == cudaSuccess) e = launch_correlations(dvel, nx, ny, zd, kCorrLinesPerChunk, scratch, dx, dy, du, s);
-    std::vector<double> h(nres);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), res, nres * sizeof(double), cudaMemcpyDeviceToHost, s);
+    cudaError_t e = cudaSuccess;
+    if (!ws) e = cudaMalloc(&own, correlations_ws(nx, ny, zd) * sizeof(double)), ws = own;
+    double *dx = ws, *dy = dx + (size_t)zd * 3 * nx, *du = dy + (size_t)zd * 3 * ny;
+    if (e == cudaSuccess) e = launch_correlations(dvel, nx, ny, zd, ws + nres, dx, dy, du, s);
+    std::vector<double> ua((size_t)zd * 3);
+    if (e == cudaSuccess && xcorl)
+        e = cudaMemcpyAsync(xcorl, dx, sizeof(double) * zd * 3 * nx, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && ycorl)
+        e = cudaMemcpyAsync(ycorl, dy, sizeof(double) * zd * 3 * ny, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ua.data(), du, sizeof(double) * zd * 3, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (scratch) cudaFree(scratch);
-    if (res) cudaFree(res);
-    if (e != cudaSuccess) return e;
-    if (xcorl) memcpy(xcorl, h.data(), sizeof(double) * zd * 3 * nx);
-    if (ycorl) memcpy(ycorl, h.data() + (size_t)zd * 3 * nx, sizeof(double) * zd * 3 * ny);
-    if (uavg)
-        for (int k = 0; k < zd; ++k) uavg[k] = h[(size_t)zd * 3 * (nx + ny) + (size_t)k * 3];
-    return cudaSuccess;
+    if (own) cudaFree(own);
+    if (e == cudaSuccess && uavg)
+        for (int k = 0; k < zd; ++k) uavg[k] = ua[(size_t)k * 3];
+    return e;
 }
 
 extern "C" int dnslbm_correlations(dnslbm_ctx *c, double *xcorl, double *ycorl, double *uavg)
@@ -1748,7 +1771,8 @@ extern "C" int dnslbm_correlations(dnslbm_ctx *c, double *xcorl, double *ycorl, 
     if (c->out_pending) CK(cudaStreamWaitEvent(c->stream, c->out_ev[1], 0));
     launch_io(c->deck.precision, 3, io_args(c), 0, c->nx, c->out_vel, c->out_den, c->stream);
     CK(cudaGetLastError());
-    const cudaError_t e = correlations_of(c->out_vel, c->nx, c->ny, zd, c->stream, xcorl, ycorl, uavg);
+    if ((rc = post_reserve(c, correlations_ws(c->nx, c->ny, zd)))) return rc;
+    const cudaError_t e = correlations_of(c->out_vel, c->nx, c->ny, zd, c->stream, c->post_ws, xcorl, ycorl, uavg);
     if (e != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "correlations: %s", cudaGetErrorString(e));
     return DNSLBM_OK;
 }
@@ -1767,7 +1791,7 @@ extern "C" int dnslbm_correlations_vel(const double *vel, int xdv, int ydv, int 
     double *dv = nullptr;
     cudaError_t e = cudaMalloc(&dv, n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemcpy(dv, vel, n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = correlations_of(dv, xdv, ydv, zd, 0, xcorl, ycorl, uavg);
+    if (e == cudaSuccess) e = correlations_of(dv, xdv, ydv, zd, 0, nullptr, xcorl, ycorl, uavg);
     if (dv) cudaFree(dv);
     if (e != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "correlations of a velocity field: %s", cudaGetErrorString(e));
     return DNSLBM_OK;
@@ -1776,20 +1800,22 @@ extern "C" int dnslbm_correlations_vel(const double *vel, int xdv, int ydv, int 
 // One-dimensional energy spectra (e-spectra/src/1d-spectra.c) of a velocity
 // field in device memory; results in the program's file layouts: ex
 // [3][nx][zd] (Euux, Evvx, Ewwx), ey [3][ny/2+1][zd] (Euuy, Evvy, Ewwy).
-static cudaError_t spectra_of(const double *dvel, int nx, int ny, int zd, cudaStream_t s, double *ex, double *ey)
+// ws as for correlations_of, of spectra_ws doubles.
+static size_t spectra_ws(int nx, int ny, int zd) { return spectra_scratch(nx, ny, zd) + (size_t)(zd - 2) * 3 * (nx + ny / 2 + 1); }
+
+static cudaError_t spectra_of(const double *dvel, int nx, int ny, int zd, cudaStream_t s, double *ws, double *ex, double *ey)
 {
     const int nj = ny / 2 + 1, nzf = zd - 2;
-    const int jb = std::max(1, std::min(8, (int)((180 * 1024) / (16 * (size_t)nx)) - 1));
-    double *scratch = nullptr, *res = nullptr;
-    const size_t nres = (size_t)nzf * 3 * (nx + nj);
-    cudaError_t e = cudaMalloc(&scratch, spectra_scratch(nx, ny, zd, jb) * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&res, nres * sizeof(double));
-    if (e == cudaSuccess) e = launch_spectra(dvel, nx, ny, zd, jb, scratch, res, res + (size_t)nzf * 3 * nx, s);
+    double *own = nullptr;
+    const size_t nres = (size_t)nzf * 3 * (nx + nj), nscr = spectra_scratch(nx, ny, zd);
+    cudaError_t e = cudaSuccess;
+    if (!ws) e = cudaMalloc(&own, spectra_ws(nx, ny, zd) * sizeof(double)), ws = own;
+    double *res = ws + nscr;  // the scratch first: its complex values want 16 bytes
+    if (e == cudaSuccess) e = launch_spectra(dvel, nx, ny, zd, ws, res, res + (size_t)nzf * 3 * nx, s);
     std::vector<double> h(nres);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), res, nres * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (scratch) cudaFree(scratch);
-    if (res) cudaFree(res);
+    if (own) cudaFree(own);
     if (e != cudaSuccess) return e;
     const double *hx = h.data(), *hy = h.data() + (size_t)nzf * 3 * nx;
     for (int c = 0; c < 3; ++c) {
@@ -1820,7 +1846,8 @@ extern "C" int dnslbm_spectra(dnslbm_ctx *c, double *ex, double *ey)
     if (c->out_pending) CK(cudaStreamWaitEvent(c->stream, c->out_ev[1], 0));
     launch_io(c->deck.precision, 3, io_args(c), 0, c->nx, c->out_vel, c->out_den, c->stream);
     CK(cudaGetLastError());
-    const cudaError_t e = spectra_of(c->out_vel, c->nx, c->ny, zd, c->stream, ex, ey);
+    if ((rc = post_reserve(c, spectra_ws(c->nx, c->ny, zd)))) return rc;
+    const cudaError_t e = spectra_of(c->out_vel, c->nx, c->ny, zd, c->stream, c->post_ws, ex, ey);
     if (e != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "spectra: %s", cudaGetErrorString(e));
     return DNSLBM_OK;
 }
@@ -1836,7 +1863,7 @@ extern "C" int dnslbm_spectra_vel(const double *vel, int xdv, int ydv, int zdv, 
     double *dv = nullptr;
     cudaError_t e = cudaMalloc(&dv, n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemcpy(dv, vel, n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = spectra_of(dv, xdv, ydv, zd, 0, ex, ey);
+    if (e == cudaSuccess) e = spectra_of(dv, xdv, ydv, zd, 0, nullptr, ex, ey);
     if (dv) cudaFree(dv);
     if (e != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "spectra of a velocity field: %s", cudaGetErrorString(e));
     return DNSLBM_OK;

@@ -259,9 +259,8 @@ int dnslbm_quadrant_vel(const double *vel, int xdv, int ydv, int zdv, int device
  * The sums are unnormalised, as the program writes them.  mean_subtract.c
  * averages over the period of a stripe texture given at compile time; its
  * shipped setting (no period) cannot run, and the plane mean here is its
- * value for any period that divides the span.  Lines up to 2048 cells;
- * temporary device memory of about 2.1 times the velocity field.  Any
- * pointer may be NULL. */
+ * value for any period that divides the span.  Lines up to 2048 cells.
+ * Any pointer may be NULL. */
 int dnslbm_correlations(dnslbm_ctx *ctx, double *xcorl, double *ycorl, double *uavg);
 /* The same for a velocity field read from a vel.NNNN file
  * ([xdv][ydv][zdv+2][3] doubles), on CUDA device `device`. */
@@ -276,7 +275,9 @@ int dnslbm_correlations_vel(const double *vel, int xdv, int ydv, int zdv, int de
  *   ey[3][ydv/2+1][zd]   Euuy, Evvy, Ewwy (per spanwise mode j),
  * the program's file layouts ([mode][zd] per component, wall planes 0).  The
  * transforms are evaluated directly in FP64 (the program calls FFTW), to
- * rounding of the DFT.  Either pointer may be NULL. */
+ * rounding of the DFT.  The workspace of the context's post-processing calls
+ * (here about 0.7 times 16 bytes per velocity value) is kept until
+ * dnslbm_destroy.  Either pointer may be NULL. */
 int dnslbm_spectra(dnslbm_ctx *ctx, double *ex, double *ey);
 /* The same for a velocity field read from a vel.NNNN file
  * ([xdv][ydv][zdv+2][3] doubles), on CUDA device `device`. */
@@ -330,12 +331,11 @@ void *dnslbm_host_alloc(size_t bytes);
 void dnslbm_host_free(void *ptr);
 
 /* Batched channels: many independent channels (own grid, walls, force,
- * state and logs) advanced together by one persistent kernel: one
- * cooperative launch runs a chunk of 32 steps (the time loop, replayed from
- * a CUDA graph), its blocks taking items of work -- runs of row groups, and
- * the cells of planes next to solids -- from a per-step counter, largest
- * first, with a bounded grid-wide barrier between steps.  All decks share
- * one precision and device.  Use dnslbm_batch_channel(b, i) with the
+ * state and logs) advanced together by one persistent kernel: one launch
+ * runs a chunk of 32 steps (the time loop, replayed from a CUDA graph), its
+ * blocks taking row groups in sequence, channel after channel; a group
+ * starts when the groups around it are done with the step before.  All decks
+ * share one precision and device.  Use dnslbm_batch_channel(b, i) with the
  * single-channel calls (flags, load/store, logs, statistics) between batch
  * steps.  The environment variable DNSLBM_BATCH=launch selects one launch
  * per step instead.  No counterpart in the reference (one channel per run). */
