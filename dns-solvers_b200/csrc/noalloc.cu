@@ -108,7 +108,11 @@ extern "C" int dnslbm_step_f64_noalloc(double *pop, size_t pop_stride, int xdv, 
     // would not fit the scratch array
     int bx = ((xdv + 31) / 32) * 32;
     if (bx > 128) bx = 128;
+    // rows a thread steps one after another: fewer where the grid would leave
+    // SMs with less than four blocks (64x32x64, ten steps: eight rows 242 us,
+    // two rows 192 us; more blocks than that only lengthen the plane sums)
     int rows = 8;
+    while (rows > 1 && (long long)((xdv + bx - 1) / bx) * ((ydv + rows - 1) / rows) * zdv < 4 * 148) rows /= 2;
     ScratchLayout L;
     for (;;) {
         const size_t nblocks = (size_t)((xdv + bx - 1) / bx) * ((ydv + rows - 1) / rows) * zdv;
