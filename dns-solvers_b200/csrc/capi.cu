@@ -580,13 +580,11 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
     // plus one; x-segmented FP64 rows: kMaxSegments groups per row)
     c->slots = std::max((int)(c->grid.x * c->grid.y), (deck->precision == 64 ? kMaxSegments : 1) * c->ny + 1);
     {
-        // Row-pipelined step.  A stage holds a group of k consecutive rows of
-        // one plane for all 19 directions.  Defaults measured on a B200
-        // (628-wide rows): two stages of about 48 KB (FP16) to 96 KB
-        // (FP32/FP64) per block; consumer threads about 2 cells each for FP64
-        // (at most 320), 3 for FP32 (at most 192), 5 for FP16 (at most 128, so
-        // two blocks share an SM).  dnslbm_autotune replaces them by measured
-        // choices; the DNSLBM_* environment variables override them.
+        // Stages hold a group of k consecutive rows of one plane for all 19
+        // directions.  Defaults measured on a B200: two stages of up to
+        // 96 KB (628x314x200 FP16, stages of 49 KB 797 us/step against 524).
+        // dnslbm_autotune replaces them by measured choices; the DNSLBM_*
+        // environment variables override them.
         const char *path = getenv("DNSLBM_PATH");
         const int row_bytes = c->pitch * (int)c->esize;
         int k = default_rows(c, row_bytes);
@@ -645,7 +643,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         {(void **)&c->d_llaunch, sizeof(LinksLaunch)},
         {(void **)&c->flow_sums, (size_t)kRing * c->nz * NP * sizeof(double)},
         {(void **)&c->flow_ctr, flow_ctr_bytes(c)},
-        {(void **)&c->flow_base, sizeof(long long)},
+        {(void **)&c->flow_base, 2 * sizeof(long long)},
     };
     for (auto &a : al) {
         cudaError_t e = cudaMalloc(a.p, a.bytes);
@@ -1164,6 +1162,7 @@ static void flow_entry(const dnslbm_ctx *c, FlowOrder o, int nsteps, unsigned fi
     L.tensor = c->maps_ok;
     L.flags = c->flow_flags;
     L.base = c->flow_base;
+    L.force_ctr = c->flow_base + 1;
     L.fpart = c->flow_part;
     L.fsums = c->flow_sums;
     L.fctr = c->flow_ctr;
@@ -2116,7 +2115,7 @@ struct dnslbm_batch {
     unsigned groups = 0;                // row groups of all channels
     unsigned *d_counter = nullptr;      // items taken
     int *d_abort = nullptr;             // a bounded wait of the launch gave up
-    int graph_ok = 1;                   // 0: stream capture of the cooperative launch was refused
+    int graph_ok = 1;                   // 0: stream capture of the launch was refused
     int withhold = 0;                   // test hook: the next run withholds a load
     unsigned long long withhold_wait_ns = 0;
     char graph_note[160] = {0};

@@ -290,8 +290,16 @@ __device__ __forceinline__ void tail_planes(const StepArgs &a, long long step, i
     }
 }
 
+// The force of the next step from the writer-side totals (encalc.c:121).
+__device__ __forceinline__ double tail_force(const StepArgs &a, double rho, double jx)
+{
+    const double N = (double)a.nx * (double)a.ny * (double)a.nz;
+    return a.const_q ? (rho / N) * a.ubulk - jx / N : a.gx;
+}
+
+// force: also set the next step's force.
 __device__ __forceinline__ void tail_record(const StepArgs &a, long long step, double force_used, int mode,
-                                            const double *plane_sums, const double (&t)[6])
+                                            const double *plane_sums, const double (&t)[6], bool force = true)
 {
     const int nz = a.nz;
     const double np = (double)a.nx * (double)a.ny;
@@ -324,7 +332,7 @@ __device__ __forceinline__ void tail_record(const StepArgs &a, long long step, d
     if (stress != stress && __ldcg(a.status) == 0) a.status[0] = step + 1;
     // constant-Q: next force from the totals of the state this step wrote
     // (encalc.c:121 evaluated one step ahead); sum of populations = t[4]
-    a.force[(step + 1) & 1] = a.const_q ? (t[4] / N) * a.ubulk - t[5] / N : a.gx;
+    if (force) a.force[(step + 1) & 1] = tail_force(a, t[4], t[5]);
 }
 
 static __device__ __forceinline__ void step_tail(const StepArgs &a, long long step, double force_used, int mode, double *smem,

@@ -525,12 +525,26 @@ __device__ __forceinline__ void flow_plane_done(const PersistArgs &a, const Chan
         if (lane == 0) persist_raise(a, s_abort);
         return;
     }
+    // constant flow rate: the next step's force first, on its own counter;
+    // the logs are off the path of the consumers that wait for it
+    if (p.const_q) {
+        double f[2] = {0.0, 0.0};
+        for (int q = lane; q < p.nz; q += 32) {
+            f[0] += __ldcg(sums + (size_t)q * NP + 6);
+            f[1] += __ldcg(sums + (size_t)q * NP + 7);
+        }
+        warp_sum<2>(f);
+        if (lane == 0) {
+            p.force[(abs_step + 1) & 1] = tail_force(p, f[0], f[1]);
+            st_release(L.force_ctr, abs_step + 1);
+        }
+    }
     double t[6] = {0, 0, 0, 0, 0, 0};
     tail_planes(p, abs_step, 0, sums, lane, 32, t);
     warp_sum<6>(t);
     __syncwarp();
     if (lane == 0) {
-        tail_record(p, abs_step, p.const_q ? __ldcg(p.force + (abs_step & 1)) : p.gx, 0, sums, t);
+        tail_record(p, abs_step, p.const_q ? __ldcg(p.force + (abs_step & 1)) : p.gx, 0, sums, t, !p.const_q);
         L.ftotal[ring] = 0;
     }
     __threadfence();
@@ -760,7 +774,7 @@ __device__ __forceinline__ void flow_consumers(const PersistArgs &a, const FlowT
         const bool q = ANYQ && p.const_q != 0;  // a launch without constant-Q channels compiles no such path
         double G = p.gx;
         if (q) {  // the force of the step: after the tail of the step before
-            if (!flow_wait_counter(a, p.step_ctr, H.abs_step, s_abort)) {
+            if (!flow_wait_counter(a, L.force_ctr, H.abs_step, s_abort)) {
                 if (lane == 0) persist_raise(a, s_abort);
                 return;
             }
@@ -796,7 +810,7 @@ __device__ __forceinline__ void flow_consumers(const PersistArgs &a, const FlowT
 static __device__ __forceinline__ void persist_reset(const ChannelLaunch &L, unsigned tid, unsigned n)
 {
     for (unsigned i = tid; i < L.flow_groups; i += n) L.flags[i] = 0;
-    if (tid == 0) *L.base = *L.p.step_ctr;
+    if (tid == 0) *L.base = *L.force_ctr = *L.p.step_ctr;
 }
 static __global__ void persist_reset_kernel(const ChannelLaunch *__restrict__ chans, int nchan, unsigned *counter)
 {

@@ -800,6 +800,7 @@ struct ChannelLaunch {
     int tensor;            // the channel's tensor maps are valid
     unsigned *flags;       // [flow_groups] steps of the launch a group is done with
     long long *base;       // step counter at the start of the launch
+    long long *force_ctr;  // steps whose force is known (constant flow rate)
     double *fpart;         // [ring][nz][gpp][NP] sums of the row groups
     double *fsums;         // [ring][nz][NP] plane sums
     unsigned *fctr;        // [ring][nz] groups of the plane done
