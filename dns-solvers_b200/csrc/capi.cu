@@ -13,6 +13,7 @@
 #include "../../include/dnslbm.h"
 #include "step_common.cuh"
 #include "step_persist.cuh"
+#include "step_batch_ordered.cuh"
 
 namespace dnslbm {
 void launch_step_f64(const StepArgs &p, dim3 grid, dim3 block, bool odd, int tex, cudaStream_t s);
@@ -78,6 +79,9 @@ static cudaError_t launch_persist_of(int precision, bool batch, const PersistArg
            : precision == 32 ? launch_persist_f32(a, groups, grid, threads, smem, any_q, links, s)
                              : launch_persist_f16(a, groups, grid, threads, smem, any_q, links, s);
 }
+int ordered_batch_occupancy(int precision, int threads, size_t smem, size_t cap);
+cudaError_t launch_ordered_batch(int precision, const ordered::PersistArgs &a, int grid, int threads, size_t smem,
+                                 cudaStream_t s);
 int tma_prepare_f64(size_t smem);
 int tma_occupancy_f64(int threads, size_t smem, bool const_q);
 void launch_tma_f64(const StepArgs &p, const TmaArgs &t, int grid, int threads, size_t smem, bool odd, int tex,
@@ -180,6 +184,7 @@ struct dnslbm_ctx {
     // channel of nz_all planes, each population array with one ghost plane
     // on either side (pop_off elements from the array's start to plane 0)
     int slab = 0, z0 = 0, nz_all = 0;
+    int plain = 0;  // rows and groups of the kernels of one launch per step: a slab, ordered_sums, or beside such a channel in a batch
     int wall_lo = 1, wall_hi = 1;
     size_t pop_off = 0;
     double *shift_all = nullptr;  // [2][nz_all][3] the channel's plane means (slab tail)
@@ -205,8 +210,19 @@ static int fail(dnslbm_ctx *c, int code, const char *fmt, ...)
         if (e_ != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
+// FP32 or FP16 with a constant flow rate: the collision takes a force rounded
+// to FP32 that is a small difference of the state's FP64 sums (1e-6 of 0.07),
+// so now and then the last bits of the sums decide the rounding, and with it
+// the roundings of the whole state.  Such a channel keeps the kernels of one
+// launch per step and their launch shapes, whose blocks sum fixed ranges of
+// rows thread by thread; the persistent kernel sums row group by row group.
+static bool ordered_sums(const dnslbm_deck &d) { return d.precision != 64 && d.force_mode == DNSLBM_FORCE_CONST_Q; }
+
 // The context steps with the persistent kernel.
-static bool uses_flow(const dnslbm_ctx *c) { return c->use_tma && !c->slab && c->tma.nseg == 1; }
+static bool uses_flow(const dnslbm_ctx *c)
+{
+    return c->use_tma && !c->slab && c->tma.nseg == 1 && !ordered_sums(c->deck);
+}
 
 // Place of population a among the arrays: in groups for the persistent
 // kernel's tensor copies, in the lattice's order otherwise.  A context changes kernels only while it holds no state.
@@ -250,7 +266,7 @@ static StepArgs step_args(const dnslbm_ctx *c)
     p.wall_lo = c->wall_lo;
     p.wall_hi = c->wall_hi;
     p.tail = c->slab ? 0 : 1;
-    p.ring = c->slab ? 0 : kRing;
+    p.ring = uses_flow(c) ? kRing : 0;
     return p;
 }
 
@@ -345,8 +361,14 @@ constexpr int kMaxSegments = 4;
 static int tma_configure(dnslbm_ctx *c, int k, int stages, int consumers, int bps, int seg = 0)
 {
     const int row_bytes = c->pitch * (int)c->esize;
-    k = std::max(1, std::min(std::min(k, c->ny), kMaxGroupRows));
-    consumers = std::max(32, std::min(c->slab || seg > 0 ? 352 : 32 * kMaxConsumerWarps, consumers / 32 * 32));
+    // whole channels step with the persistent kernel (two special warps);
+    // slabs, channels with ordered sums, and rows in x-segments, with one
+    // launch per step (one producer warp: 1256x157x100 FP64 1133 us/step
+    // against 1217 in the persistent kernel, whose stages wait longer for the
+    // edge cells' loads)
+    const bool per_step = c->slab || seg > 0 || ordered_sums(c->deck);
+    k = std::max(1, std::min(k, per_step ? c->ny : std::min(c->ny, kMaxGroupRows)));
+    consumers = std::max(32, std::min(per_step ? 352 : 32 * kMaxConsumerWarps, consumers / 32 * 32));
     if (seg > 0 && (c->deck.precision != 64 || seg % 2 || seg >= c->nx)) return -1;
     if (seg > 0) k = 1;
     const int nseg = seg > 0 ? (c->nx + seg - 1) / seg : 1;
@@ -356,11 +378,6 @@ static int tma_configure(dnslbm_ctx *c, int k, int stages, int consumers, int bp
     int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->deck.device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->deck.device);
-    // whole channels step with the persistent kernel (two special warps);
-    // slabs, and rows in x-segments, with one launch per step (one producer
-    // warp: 1256x157x100 FP64 1133 us/step against 1217 in the persistent
-    // kernel, whose stages wait longer for the edge cells' loads)
-    const bool per_step = c->slab || seg > 0;
     const size_t smem = per_step ? (size_t)stages * smem_stage + 16 * (size_t)stages : persist_smem(stages, smem_stage);
     const size_t cap = (size_t)maxsmem - kStaticSmemReserve;  // room for the kernels' static shared memory
     if (stages < 2 || smem > cap || nsm <= 0) return -1;
@@ -472,23 +489,31 @@ static cudaError_t upload_planes(dnslbm_ctx *c, const std::vector<int> *band = n
     return cudaMemcpy(c->plane_list, pl.data(), pl.size() * sizeof(int), cudaMemcpyHostToDevice);
 }
 
-// Default rows per stage group.  FP32 with a constant flow rate keeps powers of
-// two (and its consumer count): its FP32 partial sums, and through the force
-// the state's roundings, depend on which cells a thread sums.
+// Default rows per stage group.
 static int default_rows(const dnslbm_ctx *c, size_t row_bytes)
 {
-    const size_t most = c->slab && c->deck.precision == 16 ? 49152 : 98304;
+    const size_t most = c->plain && c->deck.precision == 16 ? 49152 : 98304;
     int k = 1;
-    if (c->slab || (c->deck.precision != 64 && c->deck.force_mode == DNSLBM_FORCE_CONST_Q))
+    if (c->plain)
         while (k < 8 && k * 2 <= c->ny && (size_t)Q * row_bytes * k * 2 <= most) k *= 2;
     else
         while (k < 8 && k + 1 <= c->ny && (size_t)Q * row_bytes * (k + 1) <= most) ++k;
     return k;
 }
 
+// Default consumer threads of the kernels of one launch per step: about 2
+// cells each for FP64, 3 for FP32, 5 for FP16 (two blocks share an SM).
+static int step_consumers(const dnslbm_ctx *c)
+{
+    if (const char *e = getenv("DNSLBM_THREADS")) return atoi(e) / 32 * 32;
+    const int cap = c->deck.precision == 64 ? 320 : (c->deck.precision == 32 ? 192 : 128);
+    return std::min(cap, (c->nx + 31) / 32 * 32);
+}
+
 // A whole channel (slab = 0) or the wall-normal slab [z0, z0 + nzs) of one
 // (slab = 1, dnslbm_create_slab).
-static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm_ctx **out)
+// plain: rows as for a channel with ordered sums.
+static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool plain, dnslbm_ctx **out)
 {
     dnslbm_ctx *c = nullptr;
     if (!deck || !out) return fail(c, DNSLBM_ERR_ARG, "null deck or output pointer");
@@ -523,6 +548,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
     c->ny = deck->ydv;
     c->nz = slab ? nzs : deck->zdv;
     c->slab = slab;
+    c->plain = slab || plain || ordered_sums(*deck);
     c->z0 = slab ? z0 : 0;
     c->nz_all = deck->zdv;
     c->wall_lo = c->z0 == 0;
@@ -539,7 +565,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         if (e) align_bytes = std::max(16, atoi(e));
         const int v = align_bytes / (int)c->esize;
         c->pitch = (c->nx + v - 1) / v * v;
-        if (!slab && !e && (size_t)2 * Q * c->pitch * c->esize <= (size_t)216 * 1024) {  // two whole-row stages fit
+        if (!c->plain && !e && (size_t)2 * Q * c->pitch * c->esize <= (size_t)216 * 1024) {  // two whole-row stages fit
             // rows that tensor copies can move in groups of the default size
             // (tensor_rows): up to 5 % longer
             size_t row = (size_t)c->pitch * c->esize;
@@ -592,11 +618,11 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
         int stages = 2;
         if (const char *e = getenv("DNSLBM_STAGES")) stages = atoi(e);
         // consumers: one per cell (FP64) or cell pair of a group, at most 320
-        const bool sums32 = c->deck.precision == 32 && c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
-        const int cap = slab && c->deck.precision == 16 ? 128 : ((slab || sums32) && c->deck.precision == 32 ? 192 : 320);
-        const int cells = slab || sums32 ? c->nx : (k * c->nx + (c->deck.precision != 64)) / (c->deck.precision == 64 ? 1 : 2);
-        int consumers = std::min(cap, (cells + 31) / 32 * 32);
-        if (const char *e = getenv("DNSLBM_THREADS")) consumers = atoi(e) / 32 * 32;
+        int consumers = step_consumers(c);
+        if (!c->plain && !getenv("DNSLBM_THREADS")) {
+            const int cells = c->deck.precision == 64 ? k * c->nx : (k * c->nx + 1) / 2;
+            consumers = std::min(320, (cells + 31) / 32 * 32);
+        }
         int bps = 0;
         if (const char *e = getenv("DNSLBM_BLOCKS_PER_SM")) bps = atoi(e);
         if (!(path && !strcmp(path, "scalar"))) {
@@ -690,11 +716,11 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, dnslbm
     return DNSLBM_OK;
 }
 
-extern "C" int dnslbm_create(const dnslbm_deck *deck, dnslbm_ctx **out) { return create_ctx(deck, 0, 0, 0, out); }
+extern "C" int dnslbm_create(const dnslbm_deck *deck, dnslbm_ctx **out) { return create_ctx(deck, 0, 0, 0, false, out); }
 
 extern "C" int dnslbm_create_slab(const dnslbm_deck *deck, int z0, int nzs, dnslbm_ctx **out)
 {
-    return create_ctx(deck, 1, z0, nzs, out);
+    return create_ctx(deck, 1, z0, nzs, false, out);
 }
 
 extern "C" void dnslbm_destroy(dnslbm_ctx *c)
@@ -1417,7 +1443,7 @@ extern "C" int dnslbm_set_wait_limit(dnslbm_ctx *c, double ms)
 extern "C" int dnslbm_test_withhold_load(dnslbm_ctx *c)
 {
     if (!c) return fail(c, DNSLBM_ERR_ARG, "null context");
-    if (!c->use_tma)
+    if (!c->use_tma || (!uses_flow(c) && c->tma.ngroups <= 0))
         return fail(c, DNSLBM_ERR_STATE, "the context steps with a kernel that has no bounded waits");
     c->withhold = 1;
     return DNSLBM_OK;
@@ -2064,7 +2090,8 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
         }
     }
     if (bt.k > 0 && bt.ms < best_ms) best_ms = bt.ms, best = bt.ch;  // one shape for both parities
-    if (be.k > 0 && (c->slab || be.seg > 0) && (c->slab || bo.seg > 0)) {
+    const bool per_step = c->slab || ordered_sums(c->deck);
+    if (be.k > 0 && (per_step || be.seg > 0) && (per_step || bo.seg > 0)) {
         const bool same = be.ch.threads == bo.ch.threads && be.ch.grid == bo.ch.grid && be.ch.smem == bo.ch.smem &&
                           be.ch.t.k == bo.ch.t.k && be.ch.t.stages == bo.ch.t.stages && be.ch.t.nseg == bo.ch.t.nseg;
         if (!same) {  // the parities' own shapes, measured together (a change of shape between launches costs too)
@@ -2119,6 +2146,18 @@ struct dnslbm_batch {
     int withhold = 0;                   // test hook: the next run withholds a load
     unsigned long long withhold_wait_ns = 0;
     char graph_note[160] = {0};
+    // some channel has ordered sums: the persistent kernel of
+    // step_batch_ordered.cuh, its blocks taking items of work from a
+    // per-step counter
+    int ordered = 0;
+    std::vector<ordered::BatchItem> items;  // the items of one step, largest first
+    int items_per_block = 4;                // items per resident block and step the items are cut for
+    std::vector<ordered::BatchItem> items_uploaded;
+    ordered::BatchItem *d_items = nullptr;
+    size_t d_items_cap = 0;
+    unsigned *d_counters = nullptr;         // [graph_steps] items taken per step
+    unsigned *d_arrivals = nullptr;         // grid-barrier arrivals
+    bool flow() const { return persistent && !ordered; }  // the persistent kernel of step_persist.cuh
     size_t budget = 0;  // shared-memory budget per block the stages were sized for
     int stages = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -2168,6 +2207,9 @@ extern "C" void dnslbm_batch_destroy(dnslbm_batch *b)
     if (b->d_maps) cudaFree(b->d_maps);
     if (b->d_counter) cudaFree(b->d_counter);
     if (b->d_abort) cudaFree(b->d_abort);
+    if (b->d_items) cudaFree(b->d_items);
+    if (b->d_counters) cudaFree(b->d_counters);
+    if (b->d_arrivals) cudaFree(b->d_arrivals);
     for (auto &e : b->fj)
         if (e) cudaEventDestroy(e);
     if (b->side) cudaStreamDestroy(b->side);
@@ -2179,13 +2221,18 @@ extern "C" void dnslbm_batch_destroy(dnslbm_batch *b)
 // Shared-memory budgets per block for one, two and three blocks per SM
 // (228 KB per SM, 1 KB of it reserved per block, the static shared memory of
 // the kernel on top).
-constexpr size_t kBatchBudget1 = 220 * 1024, kBatchBudget2 = 112 * 1024, kBatchBudget3 = 70 * 1024;
+// The kernels of step_tma.cuh and step_batch_ordered.cuh have more static
+// shared memory.
+constexpr size_t kBatchBudget1 = 220 * 1024, kBatchBudget3 = 70 * 1024;
+static size_t batch_budget2(const dnslbm_batch *b) { return (b->flow() ? 112 : 108) * 1024; }
 
 // Row groups of every channel's planes without link masks shared among the
 // resident blocks, each block taking whole row groups of one channel and
 // about the same number of cells, and the block count of the per-cell pass
 // over the planes with link masks.  A change of
 // either grid invalidates the captured graphs.
+static void ordered_items(dnslbm_batch *b);
+
 static void batch_layout(dnslbm_batch *b)
 {
     // a common amount of work per block (cells of whole row groups), the
@@ -2227,6 +2274,52 @@ static void batch_layout(dnslbm_batch *b)
     b->nlinks = nl;
     if ((nl > 0) != (b->any_links != 0)) destroy_graphs(b);  // another form of the persistent kernel
     b->any_links = nl > 0;
+    if (b->persistent && b->ordered) ordered_items(b);
+}
+
+// The items of one step of a batch with ordered sums: each plane of each
+// channel cut into runs of whole row groups of about W cells, W chosen so
+// that every resident block takes about items_per_block items per step (more
+// and smaller items even out the blocks' ends of a step, at a cost per
+// item; the batch autotuner picks the count); kind 1 for the
+// planes with link masks (the channel's plane list holds them after the
+// others, so the group numbering covers them).  Largest first, so the last
+// items taken are the small ones.  An item's slot is its index within its
+// plane, so the plane sums do not depend on which block takes it.
+static void ordered_items(dnslbm_batch *b)
+{
+    double total = 0;
+    for (auto *c : b->ch) total += (double)c->nx * c->ny * c->nz;
+    const double W = std::max(1.0, total / ((double)b->items_per_block * std::max(1, b->pgrid)));
+    std::vector<ordered::BatchItem> it;
+    std::vector<double> cells;
+    for (int ci = 0; ci < (int)b->ch.size(); ++ci) {
+        dnslbm_ctx *c = b->ch[ci];
+        const TmaArgs &t = c->tma;
+        for (int pi = 0; pi < c->nz; ++pi) {
+            const double gcells = (double)t.k * c->nx;
+            const int per = std::max(1, (int)(W / gcells));
+            const int n = (t.gpp + per - 1) / per;
+            for (int j = 0; j < n; ++j) {
+                const int g0 = (int)((long long)t.gpp * j / n), g1 = (int)((long long)t.gpp * (j + 1) / n);
+                ordered::BatchItem x{};
+                x.chan = ci;
+                x.kind = pi < c->nclean ? 0 : 1;
+                x.first = pi * t.gpp + g0;
+                x.count = g1 - g0;
+                x.plane = c->plane_host[pi];
+                x.slot = j;
+                x.ncontrib = n;
+                it.push_back(x);
+                cells.push_back(std::min((double)(g1 - g0) * t.k, (double)c->ny) * c->nx);
+            }
+        }
+    }
+    std::vector<int> order(it.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cells[a] > cells[c]; });
+    b->items.resize(it.size());
+    for (size_t i = 0; i < order.size(); ++i) b->items[i] = it[order[i]];
 }
 
 // Shape of the persistent kernel for the current stages and consumers:
@@ -2260,6 +2353,50 @@ static int persist_configure(dnslbm_batch *b)
     return 0;
 }
 
+// The same of the kernel with ordered sums.
+static int ordered_configure(dnslbm_batch *b)
+{
+    size_t stage = 0;
+    for (auto *c : b->ch) stage = std::max(stage, (size_t)Q * c->tma.row_bytes * c->tma.k);
+    const size_t smem = ordered::persist_smem(b->stages, stage);
+    int maxsmem = 0, nsm = 0;
+    cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
+    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
+    if (smem > cap || nsm < 1) return -1;
+    const int occ = ordered_batch_occupancy(b->precision, b->threads, smem, cap);
+    cudaGetLastError();
+    if (occ < 1) return -1;
+    b->pstage = stage;
+    b->psmem = smem;
+    b->pgrid = occ * nsm;
+    return 0;
+}
+
+// The shape of a channel of a batch when it is stepped by itself by the
+// persistent kernel of one channel: the batch's stages and consumers, its own
+// stage size.
+static int member_shape(dnslbm_ctx *c, int stages, int consumers)
+{
+    const int threads = std::min(consumers, 32 * kMaxConsumerWarps) + 64;
+    const size_t smem = persist_smem(stages, (size_t)Q * c->tma.dir_elems * c->esize);
+    int maxsmem = 0, nsm = 0;
+    cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->deck.device);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->deck.device);
+    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
+    const bool q = c->deck.force_mode == DNSLBM_FORCE_CONST_Q, general = c->deck.bc_mode == DNSLBM_BC_GENERAL;
+    if (smem > cap || persist_prepare(c->deck.precision, false, threads, cap, q, false) ||
+        (general && persist_prepare(c->deck.precision, false, threads, cap, q, true)))
+        return -1;
+    const int occ = persist_occupancy_of(c->deck.precision, false, threads, smem, q, general);
+    cudaGetLastError();
+    if (occ < 1) return -1;
+    c->tma_threads = threads;
+    c->tma_smem = smem;
+    c->tma_target = occ * nsm;
+    return 0;
+}
+
 // One launch shape for all channels: per channel the most rows per stage
 // group (up to 16) whose `stages` groups fit `budget` bytes, so channels of
 // short rows move about as many bytes per stage as those of long rows; the
@@ -2267,22 +2404,23 @@ static int persist_configure(dnslbm_batch *b)
 // when it runs on the device.
 static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consumers)
 {
-    const int special = b->persistent ? 64 : 32;  // threads of the load and store warps, or of the producer
-    consumers = std::max(32, std::min(b->persistent ? 32 * kMaxConsumerWarps : 352, consumers / 32 * 32));
+    const bool flow = b->flow();
+    const int special = flow ? 64 : 32;  // threads of the load and store warps, or of the producer
+    consumers = std::max(32, std::min(flow ? 32 * kMaxConsumerWarps : 352, consumers / 32 * 32));
     size_t smem = 0;
     std::vector<int> ks(b->ch.size());
     for (size_t i = 0; i < b->ch.size(); ++i) {
         dnslbm_ctx *c = b->ch[i];
         const int row_bytes = c->pitch * (int)c->esize;
         auto need = [&](int k) {
-            return b->persistent ? persist_smem(stages, (size_t)Q * row_bytes * k, (int)b->ch.size())
-                                 : (size_t)stages * Q * row_bytes * k + 16 * (size_t)stages;
+            return flow ? persist_smem(stages, (size_t)Q * row_bytes * k, (int)b->ch.size())
+                        : (size_t)stages * Q * row_bytes * k + 16 * (size_t)stages;
         };
         if (need(1) > budget) return -1;
         int k = 1;
         while (k < 16 && k + 1 <= c->ny && need(k + 1) <= budget) ++k;
         // a size that tensor copies take, if one is near
-        if (b->persistent)
+        if (flow)
             for (int q = k; q >= 1 && 4 * q >= 3 * k; --q)
                 if (tensor_rows((size_t)row_bytes, q)) {
                     k = q;
@@ -2298,7 +2436,7 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
     const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
     if (smem > cap || nsm < 1) return -1;
     int occ = 1;
-    if (!b->persistent) {
+    if (!flow) {
         const int prep = b->precision == 64 ? tma_batch_prepare_f64(cap) : tma_batch_prepare_lp(b->precision, cap);
         occ = prep ? 0
                    : (b->precision == 64 ? tma_batch_occupancy_f64(threads, smem)
@@ -2321,7 +2459,11 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
     b->smem = smem;
     b->budget = budget;
     b->stages = stages;
-    if (b->persistent) {
+    if (b->persistent && b->ordered) {
+        if (ordered_configure(b)) return -1;
+        for (auto *c : b->ch)
+            if (uses_flow(c) && member_shape(c, stages, consumers)) return -1;
+    } else if (flow) {
         if (persist_configure(b)) return -1;
         for (auto *c : b->ch) {  // what a channel stepped by itself takes: the same stages, its own stage size
             c->tma_smem = persist_smem(stages, (size_t)Q * c->tma.dir_elems * c->esize);
@@ -2351,9 +2493,10 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
     // DNSLBM_BATCH=launch: one launch of the per-step batch kernel per step
     // (the layout before the persistent kernel, kept for comparison)
     if (const char *e = getenv("DNSLBM_BATCH")) b->persistent = strcmp(e, "launch") != 0;
+    for (int i = 0; i < n; ++i) b->ordered |= ordered_sums(decks[i]);
     for (int i = 0; i < n; ++i) {
         dnslbm_ctx *c = nullptr;
-        int rc = dnslbm_create(&decks[i], &c);
+        int rc = create_ctx(&decks[i], 0, 0, 0, b->ordered != 0, &c);
         if (rc) {
             char msg[512];
             snprintf(msg, sizeof msg, "channel %d: %s", i, g_create_err);
@@ -2376,11 +2519,13 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
     };
     if (cudaSetDevice(b->device) != cudaSuccess) return bail(bfail(b, DNSLBM_ERR_CUDA, "cannot select device"));
     b->maps_k.assign(n, 0);
-    // default launch shape: stages sized for two blocks per SM, the widest
-    // consumer set any channel would use alone
+    // default launch shape: two stages, sized for one block per SM (two in the
+    // kernels of step_tma.cuh and step_batch_ordered.cuh), the widest consumer
+    // set any channel would use alone
     int consumers = 32;
-    for (auto *c : b->ch) consumers = std::max(consumers, c->tma_threads - 64);
-    if (batch_configure(b, kBatchBudget1, 2, consumers) && batch_configure(b, kBatchBudget2, 2, consumers))
+    for (auto *c : b->ch) consumers = std::max(consumers, b->flow() ? c->tma_threads - 64 : step_consumers(c));
+    const size_t budgets[2] = {kBatchBudget1, batch_budget2(b)};
+    if (batch_configure(b, budgets[!b->flow()], 2, consumers) && batch_configure(b, budgets[b->flow()], 2, consumers))
         return bail(bfail(b, DNSLBM_ERR_ARG, "batched kernel does not fit the device"));
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess ||
@@ -2391,6 +2536,8 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
         cudaEventCreateWithFlags(&b->fj[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(&b->d_flow, sizeof(ChannelLaunch) * 2 * n) != cudaSuccess ||
         cudaMalloc(&b->d_counter, sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&b->d_counters, sizeof(unsigned) * b->graph_steps) != cudaSuccess ||
+        cudaMalloc(&b->d_arrivals, sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&b->d_maps, sizeof(FlowMaps) * n) != cudaSuccess ||
         cudaMalloc(&b->d_abort, sizeof(int)) != cudaSuccess || cudaMemset(b->d_abort, 0, sizeof(int)) != cudaSuccess)
         return bail(bfail(b, DNSLBM_ERR_CUDA, "batch set-up failed: %s", cudaGetErrorString(cudaGetLastError())));
@@ -2452,6 +2599,51 @@ static int persist_launch(dnslbm_batch *b, int n, int slot)
     return DNSLBM_OK;
 }
 
+// The same of the kernel with ordered sums, from parity `odd`: counters and
+// barrier arrivals cleared, then one cooperative launch.
+static int ordered_launch(dnslbm_batch *b, int n, int odd)
+{
+    ordered::PersistArgs a;
+    a.chans = b->d_launch;
+    a.items = b->d_items;
+    a.nitems = (int)b->items.size();
+    a.nsteps = n;
+    a.first_odd = odd;
+    a.stages = b->stages;
+    a.stage_bytes = (unsigned)b->pstage;
+    a.counters = b->d_counters;
+    a.arrivals = b->d_arrivals;
+    a.abort = b->d_abort;
+    a.wait_ns = b->withhold ? b->withhold_wait_ns : b->ch[0]->wait_ns;
+    a.withhold = b->withhold;
+    BCK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned) * n, b->stream));
+    BCK(cudaMemsetAsync(b->d_arrivals, 0, sizeof(unsigned), b->stream));
+    BCK(launch_ordered_batch(b->precision, a, b->pgrid, b->threads, b->psmem, b->stream));
+    return DNSLBM_OK;
+}
+
+// Its item table on the device (a new one invalidates the captured graphs,
+// which hold its address and length).
+static int ordered_upload(dnslbm_batch *b)
+{
+    if (b->items.size() > b->d_items_cap) {
+        if (b->d_items) cudaFree(b->d_items);
+        b->d_items = nullptr;
+        b->d_items_cap = 0;
+        BCK(cudaMalloc(&b->d_items, sizeof b->items[0] * b->items.size()));
+        b->d_items_cap = b->items.size();
+        destroy_graphs(b);
+    }
+    if (b->items.size() != b->items_uploaded.size() ||
+        memcmp(b->items.data(), b->items_uploaded.data(), sizeof b->items[0] * b->items.size())) {
+        destroy_graphs(b);
+        b->items_uploaded = b->items;
+    }
+    BCK(cudaMemcpyAsync(b->d_items, b->items.data(), sizeof b->items[0] * b->items.size(), cudaMemcpyHostToDevice,
+                        b->stream));
+    return DNSLBM_OK;
+}
+
 // The launch table of n steps: the channels one after another, each through
 // all n steps (a small one stays in L2), the blocks moving on to the next
 // channel as they run out of items.
@@ -2487,19 +2679,22 @@ static int persist_run(dnslbm_batch *b, long nsteps)
     BCK(cudaMemsetAsync(b->d_abort, 0, sizeof(int), b->stream));
     double groups = 0;
     for (auto *c : b->ch) groups += (double)c->tma.gpp * c->nz;
-    const int chunk = std::min(b->graph_steps, flow_chunk(groups));
+    const int chunk = b->flow() ? std::min(b->graph_steps, flow_chunk(groups)) : b->graph_steps;
+    int odd = b->ch[0]->odd;
     while (left > 0) {
         const int n = (int)std::min<long>(left, chunk), slot = n == chunk ? 0 : 1;
-        if (int rc = persist_table(b, n, slot)) return rc;
+        if (b->flow())
+            if (int rc = persist_table(b, n, slot)) return rc;
+        auto launch = [&]() { return b->flow() ? persist_launch(b, n, slot) : ordered_launch(b, n, odd); };
         if (slot == 0 && b->graph_ok && !b->withhold) {
-            cudaGraphExec_t &g = b->graph[0];
+            cudaGraphExec_t &g = b->graph[b->flow() ? 0 : odd];
             if (!g) {
                 // the time loop's chunk captured as a graph; a driver that
                 // refuses to capture the launch leaves plain launches (noted
                 // in the kernel description)
                 cudaGraph_t graph = nullptr;
                 BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-                const int rc = persist_launch(b, n, slot);
+                const int rc = launch();
                 cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
                 if (rc == DNSLBM_OK && ee == cudaSuccess) ee = cudaGraphInstantiate(&g, graph, 0);
                 if (graph) cudaGraphDestroy(graph);
@@ -2514,11 +2709,12 @@ static int persist_run(dnslbm_batch *b, long nsteps)
             }
             BCK(cudaGraphLaunch(g, b->stream));
         } else {
-            const int rc = persist_launch(b, n, slot);
+            const int rc = launch();
             b->withhold = 0;
             if (rc) return rc;
         }
         left -= n;
+        odd = (odd + n) & 1;
     }
     return DNSLBM_OK;
 }
@@ -2564,6 +2760,8 @@ static int batch_run(dnslbm_batch *b, long nsteps, double *ms)
     if (!hl.empty())
         BCK(cudaMemcpyAsync(b->d_links, hl.data(), sizeof(LinksLaunch) * hl.size(), cudaMemcpyHostToDevice,
                             b->stream));
+    if (b->persistent && b->ordered)
+        if (int rc = ordered_upload(b)) return rc;
     int odd = b->ch[0]->odd;
     long left = nsteps;
     if (ms) BCK(cudaEventRecord(b->ev[0], b->stream));
@@ -2650,6 +2848,14 @@ extern "C" const char *dnslbm_batch_kernel(const dnslbm_batch *b)
 {
     static thread_local char buf[384];
     if (!b) return "";
+    if (b->persistent && b->ordered) {
+        snprintf(buf, sizeof buf,
+                 "persist_batch_kernel<fp%d> with ordered sums: %zu channels, %zu items per step, %d blocks x %d threads, "
+                 "%d stages, %zu B smem; one cooperative launch per %d steps, CUDA graph%s",
+                 b->precision, b->ch.size(), b->items.size(), b->pgrid, b->threads, b->stages, b->psmem, b->graph_steps,
+                 b->graph_note);
+        return buf;
+    }
     if (b->persistent) {
         snprintf(buf, sizeof buf,
                  "persist_batch_kernel<fp%d>: %zu channels, %d blocks x %d threads, %d stages, %zu B smem; one launch "
@@ -2674,9 +2880,9 @@ extern "C" int dnslbm_batch_autotune(dnslbm_batch *b, int steps, char *report, s
     if (steps >= b->graph_steps) steps = b->graph_steps - 1;  // plain launches, no graph to capture
     BCK(cudaSetDevice(b->device));
     size_t bb = b->budget;
-    int bs = b->stages, bc = b->threads - (b->persistent ? 64 : 32), ncand = 0;
+    int bs = b->stages, bc = b->threads - (b->flow() ? 64 : 32), ncand = 0;
     double best = 1e30;
-    for (size_t budget : {kBatchBudget1, kBatchBudget2, kBatchBudget3})
+    for (size_t budget : {kBatchBudget1, batch_budget2(b), kBatchBudget3})
         for (int st : {2, 3, 4})
             for (int cons : {64, 128, 192, 256, 320}) {
                 if (batch_configure(b, budget, st, cons)) continue;
@@ -2688,6 +2894,22 @@ extern "C" int dnslbm_batch_autotune(dnslbm_batch *b, int steps, char *report, s
                 ++ncand;
                 if (ms < best) best = ms, bb = budget, bs = st, bc = cons;
             }
+    // ordered sums: how finely each step's work is cut, at the best shape
+    if (b->persistent && b->ordered) {
+        int bi = b->items_per_block;
+        for (int ipb : {2, 8, 16}) {
+            b->items_per_block = ipb;
+            if (batch_configure(b, bb, bs, bc)) continue;
+            int rc = DNSLBM_OK;
+            for (auto *c : b->ch)
+                if ((rc = dnslbm_init_rest(c))) return bfail(b, rc, "%s", c->err);
+            double ms = 0;
+            if ((rc = batch_run(b, 2, nullptr)) || (rc = batch_run(b, steps, &ms))) return rc;
+            ++ncand;
+            if (ms < best) best = ms, bi = ipb;
+        }
+        b->items_per_block = bi;
+    }
     // leave the channels as created: no state, counters clear
     for (auto *c : b->ch) {
         int rc = reset_counters(c);
