@@ -1204,6 +1204,11 @@ static int flow_eager(double groups, int blocks, int stages) { return groups < 4
 
 static int flow_steps(dnslbm_ctx *c, long n)
 {
+    const size_t stage_bytes = (size_t)Q * c->tma.dir_elems * c->esize;
+    // the kernel's own layout: two special warps, and barriers, sums and headers behind the stages
+    if (c->tma_threads < 96 || c->tma_smem < persist_smem(c->tma.stages, stage_bytes))
+        return fail(c, DNSLBM_ERR_STATE, "%d threads and %zu bytes are not a launch shape of the persistent kernel",
+                    c->tma_threads, c->tma_smem);
     if (int rc = flow_reserve(c)) return rc;
     flow_maps(c);
     const FlowOrder o = flow_order(c, c->tma_target);
@@ -1213,7 +1218,7 @@ static int flow_steps(dnslbm_ctx *c, long n)
     PersistArgs a{};
     a.nchan = 1;
     a.stages = c->tma.stages;
-    a.stage_bytes = (unsigned)((size_t)Q * c->tma.dir_elems * c->esize);
+    a.stage_bytes = (unsigned)stage_bytes;
     a.counter = c->flow_ctr + (size_t)kRing * (c->nz + 1);
     a.abort = reinterpret_cast<int *>(c->status + 1);
     a.wait_ns = c->wait_ns;
@@ -2459,11 +2464,11 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
     b->smem = smem;
     b->budget = budget;
     b->stages = stages;
-    if (b->persistent && b->ordered) {
-        if (ordered_configure(b)) return -1;
+    if (!flow) {
+        if (b->persistent && ordered_configure(b)) return -1;
         for (auto *c : b->ch)
             if (uses_flow(c) && member_shape(c, stages, consumers)) return -1;
-    } else if (flow) {
+    } else {
         if (persist_configure(b)) return -1;
         for (auto *c : b->ch) {  // what a channel stepped by itself takes: the same stages, its own stage size
             c->tma_smem = persist_smem(stages, (size_t)Q * c->tma.dir_elems * c->esize);
