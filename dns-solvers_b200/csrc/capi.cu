@@ -136,7 +136,7 @@ struct dnslbm_ctx {
     double *flow_part = nullptr;      // [kRing][row groups][NP]
     size_t flow_part_n = 0;
     double *flow_sums = nullptr;      // [kRing][nz][NP]
-    unsigned *flow_ctr = nullptr;     // [kRing][nz] groups done, [kRing] planes done, the item counter
+    unsigned *flow_ctr = nullptr;     // [kRing][nz] groups done, [kRing] planes done, the items and planes taken
     long long *flow_base = nullptr;
     double *force = nullptr, *shift = nullptr, *partials = nullptr, *plane_sums = nullptr, *logs = nullptr;
     long long *step_ctr = nullptr, *status = nullptr;
@@ -176,6 +176,7 @@ struct dnslbm_ctx {
     int have_state = 0;
     unsigned long long wait_ns = 1000000000ull;  // limit of a bounded device wait (1 s)
     int withhold = 0;                            // test hook: the next bulk-copy launch withholds a load
+    int test_blocks = 0;                         // test hook: blocks of the persistent kernel's launches, 0: the launch shape's
     int odd = 0;  // parity of the next step (1: populations are post-collision, swapped)
     long long done = 0;
     int slab_next = 0;  // next x of a state loaded in slabs
@@ -284,7 +285,7 @@ static int row_pieces(size_t row_bytes)
 static bool tensor_rows(size_t row_bytes, int k) { return row_pieces(row_bytes) > 0 && row_bytes * k % 128 == 0; }
 
 static size_t shift_bytes(const dnslbm_ctx *c) { return (size_t)(c->slab ? 2 : kRing) * c->nz * 3 * sizeof(double); }
-static size_t flow_ctr_bytes(const dnslbm_ctx *c) { return ((size_t)kRing * (c->nz + 1) + 1) * sizeof(unsigned); }
+static size_t flow_ctr_bytes(const dnslbm_ctx *c) { return ((size_t)kRing * (c->nz + 1) + 2) * sizeof(unsigned); }
 
 static IoArgs io_args(const dnslbm_ctx *c)
 {
@@ -1232,8 +1233,9 @@ static int flow_steps(dnslbm_ctx *c, long n)
         a.nsteps = m;
         a.withhold = c->withhold;
         c->withhold = 0;
-        CK(launch_persist_of(c->deck.precision, false, a, groups, (int)std::min<unsigned>(c->tma_target, L.item_end),
-                                c->tma_threads, c->tma_smem, L.p.const_q != 0, c->ndirty > 0, c->stream));
+        const int grid = c->test_blocks ? c->test_blocks : (int)std::min<unsigned>(c->tma_target, L.item_end);
+        CK(launch_persist_of(c->deck.precision, false, a, groups, grid, c->tma_threads,
+                             c->tma_smem, L.p.const_q != 0, c->ndirty > 0, c->stream));
         c->odd = (c->odd + m) & 1;
         c->done += m;
         n -= m;
@@ -1451,6 +1453,14 @@ extern "C" int dnslbm_test_withhold_load(dnslbm_ctx *c)
     if (!c->use_tma || (!uses_flow(c) && c->tma.ngroups <= 0))
         return fail(c, DNSLBM_ERR_STATE, "the context steps with a kernel that has no bounded waits");
     c->withhold = 1;
+    return DNSLBM_OK;
+}
+
+extern "C" int dnslbm_test_blocks(dnslbm_ctx *c, int blocks)
+{
+    if (!c || blocks < 0 || blocks > 65535) return fail(c, DNSLBM_ERR_ARG, "null context or %d blocks", blocks);
+    if (!uses_flow(c)) return fail(c, DNSLBM_ERR_STATE, "the context does not step with the persistent kernel");
+    c->test_blocks = blocks;
     return DNSLBM_OK;
 }
 
@@ -2145,7 +2155,7 @@ struct dnslbm_batch {
     FlowMaps *d_maps = nullptr;         // [n] the channels' tensor maps
     std::vector<int> maps_k;            // rows of the groups they are for
     unsigned groups = 0;                // row groups of all channels
-    unsigned *d_counter = nullptr;      // items taken
+    unsigned *d_counter = nullptr;      // items and planes taken
     int *d_abort = nullptr;             // a bounded wait of the launch gave up
     int graph_ok = 1;                   // 0: stream capture of the launch was refused
     int withhold = 0;                   // test hook: the next run withholds a load
@@ -2540,7 +2550,7 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
         cudaEventCreateWithFlags(&b->fj[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->fj[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(&b->d_flow, sizeof(ChannelLaunch) * 2 * n) != cudaSuccess ||
-        cudaMalloc(&b->d_counter, sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&b->d_counter, 2 * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&b->d_counters, sizeof(unsigned) * b->graph_steps) != cudaSuccess ||
         cudaMalloc(&b->d_arrivals, sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&b->d_maps, sizeof(FlowMaps) * n) != cudaSuccess ||

@@ -88,6 +88,7 @@ def lib():
     L.dnslbm_output_wait.argtypes = [vp]
     L.dnslbm_set_wait_limit.argtypes = [vp, ctypes.c_double]
     L.dnslbm_test_withhold_load.argtypes = [vp]
+    L.dnslbm_test_blocks.argtypes = [vp, ctypes.c_int]
     L.dnslbm_step_kernel.argtypes = [vp]
     L.dnslbm_step_kernel.restype = ctypes.c_char_p
     L.dnslbm_bytes_per_cell.argtypes = [vp]
@@ -268,6 +269,11 @@ class Channel:
         """Test hook: the next bulk-copy launch withholds one load, so a
         bounded wait runs out and that step call raises ERR_TIMEOUT."""
         self._ck(self.L.dnslbm_test_withhold_load(self.h))
+
+    def test_blocks(self, blocks: int):
+        """Test hook: blocks of the persistent kernel's launches (0: its own
+        number)."""
+        self._ck(self.L.dnslbm_test_blocks(self.h, blocks))
 
     @property
     def steps_done(self):

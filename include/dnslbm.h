@@ -315,6 +315,11 @@ int dnslbm_set_wait_limit(dnslbm_ctx *ctx, double ms);
  * DNSLBM_ERR_TIMEOUT.  Nothing faults and no copy is left in flight.
  * DNSLBM_ERR_STATE when the context steps with the per-thread kernel. */
 int dnslbm_test_withhold_load(dnslbm_ctx *ctx);
+/* Test hook (no counterpart in the reference): the persistent kernel is
+ * launched with this many blocks, fewer or more than the GPU holds at once
+ * (0: its own number).  The results do not depend on it.  DNSLBM_ERR_STATE
+ * when the context steps with another kernel. */
+int dnslbm_test_blocks(dnslbm_ctx *ctx, int blocks);
 
 /* Name of the step kernel this context launches ("row-pipelined bulk-copy"
  * or "per-thread"), with its launch shape. */
