@@ -336,6 +336,8 @@ extern "C" const char *dnslbm_last_error(const dnslbm_ctx *c) { return c ? c->er
 // Dynamic shared memory the step kernels may be given: the device's opt-in
 // maximum less this reserve for their static shared memory (about 2.5 KB).
 constexpr size_t kStaticSmemReserve = 4096;
+// The same of the persistent kernel (128 bytes).
+constexpr size_t kPersistSmemReserve = 1024;
 
 // Row groups of the row-pipelined kernel over its planes (all planes, or the
 // planes without link masks) shared among tma_target blocks.
@@ -380,7 +382,7 @@ static int tma_configure(dnslbm_ctx *c, int k, int stages, int consumers, int bp
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->deck.device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->deck.device);
     const size_t smem = per_step ? (size_t)stages * smem_stage + 16 * (size_t)stages : persist_smem(stages, smem_stage);
-    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;  // room for the kernels' static shared memory
+    const size_t cap = (size_t)maxsmem - (per_step ? kStaticSmemReserve : kPersistSmemReserve);
     if (stages < 2 || smem > cap || nsm <= 0) return -1;
     const int threads = consumers + (per_step ? 32 : 64);
     const bool const_q = c->deck.force_mode == DNSLBM_FORCE_CONST_Q;
@@ -2344,11 +2346,11 @@ static int persist_configure(dnslbm_batch *b)
     size_t stage = 0;
     for (auto *c : b->ch) stage = std::max(stage, (size_t)Q * c->tma.row_bytes * c->tma.k);
     stage = (stage + 127) / 128 * 128;  // tensor copies land on 128 bytes
-    const size_t smem = persist_smem(b->stages, stage, (int)b->ch.size());
+    const size_t smem = persist_smem(b->stages, stage, true);
     int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
-    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
+    const size_t cap = (size_t)maxsmem - kPersistSmemReserve;
     if (smem > cap || nsm < 1) return -1;
     b->any_q = 0;
     b->general = 0;
@@ -2398,7 +2400,7 @@ static int member_shape(dnslbm_ctx *c, int stages, int consumers)
     int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->deck.device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->deck.device);
-    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
+    const size_t cap = (size_t)maxsmem - kPersistSmemReserve;
     const bool q = c->deck.force_mode == DNSLBM_FORCE_CONST_Q, general = c->deck.bc_mode == DNSLBM_BC_GENERAL;
     if (smem > cap || persist_prepare(c->deck.precision, false, threads, cap, q, false) ||
         (general && persist_prepare(c->deck.precision, false, threads, cap, q, true)))
@@ -2428,7 +2430,7 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
         dnslbm_ctx *c = b->ch[i];
         const int row_bytes = c->pitch * (int)c->esize;
         auto need = [&](int k) {
-            return flow ? persist_smem(stages, (size_t)Q * row_bytes * k, (int)b->ch.size())
+            return flow ? persist_smem(stages, (size_t)Q * row_bytes * k, true)
                         : (size_t)stages * Q * row_bytes * k + 16 * (size_t)stages;
         };
         if (need(1) > budget) return -1;
@@ -2448,7 +2450,7 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
     int maxsmem = 0, nsm = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
-    const size_t cap = (size_t)maxsmem - kStaticSmemReserve;
+    const size_t cap = (size_t)maxsmem - (flow ? kPersistSmemReserve : kStaticSmemReserve);
     if (smem > cap || nsm < 1) return -1;
     int occ = 1;
     if (!flow) {
@@ -2540,7 +2542,10 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
     int consumers = 32;
     for (auto *c : b->ch) consumers = std::max(consumers, b->flow() ? c->tma_threads - 64 : step_consumers(c));
     const size_t budgets[2] = {kBatchBudget1, batch_budget2(b)};
-    if (batch_configure(b, budgets[!b->flow()], 2, consumers) && batch_configure(b, budgets[b->flow()], 2, consumers))
+    int maxsmem = 0;  // the longest rows want all there is
+    cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+    if (batch_configure(b, budgets[!b->flow()], 2, consumers) && batch_configure(b, budgets[b->flow()], 2, consumers) &&
+        (!b->flow() || batch_configure(b, (size_t)maxsmem - kPersistSmemReserve, 2, consumers)))
         return bail(bfail(b, DNSLBM_ERR_ARG, "batched kernel does not fit the device"));
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess ||

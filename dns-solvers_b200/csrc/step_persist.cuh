@@ -149,33 +149,56 @@ struct StageHeader {
 constexpr int kMaxConsumerWarps = kTmaMaxThreads / 32 - 2;
 
 // Where the warps read the channels' arguments: the kernel's parameters for
-// one channel, a copy of the table in shared memory for a batch.  (The
+// one channel; for a batch, copies in shared memory of the table's entries in
+// use -- one per stage, the load warp's, and the store warp's for the plane it
+// looks after -- so that the number of channels costs none of it.  (The
 // acquiring loads of the flags drop the SM's L1 contents again and again, so
-// a table in global memory would come from L2 every time.)
+// an entry in global memory would come from L2 every time.)
+constexpr int kEntries = 2;  // besides the stages'
 template <bool ONE>
 struct FlowTable {
     const PersistArgs &a;
-    const ChannelLaunch *table;
-    __device__ __forceinline__ const ChannelLaunch &operator[](int c) const
+    ChannelLaunch *copies;  // the load warp's, the store warp's, [stages]
+    __device__ __forceinline__ const ChannelLaunch &load() const { return at(0); }
+    __device__ __forceinline__ const ChannelLaunch &duty() const { return at(1); }
+    __device__ __forceinline__ const ChannelLaunch &stage(int st) const { return at(kEntries + st); }
+    __device__ __forceinline__ const ChannelLaunch &at(int i) const
     {
         if constexpr (ONE) return a.one;
-        else return table[c];
+        else return copies[i];
     }
     __device__ __forceinline__ int count() const { return ONE ? 1 : a.nchan; }
+    // entry c of the table in global memory
+    __device__ __forceinline__ const ChannelLaunch &entry(int c) const
+    {
+        if constexpr (ONE) return a.one;
+        else return a.chans[c];
+    }
     __device__ __forceinline__ const FlowMaps &maps(int c) const
     {
         if constexpr (ONE) return a.one_maps;
         else return a.maps[c];
     }
+    // copy i of entry c, by the whole warp that uses it
+    __device__ __forceinline__ void fetch(int i, int c, int lane) const
+    {
+        if constexpr (!ONE) {
+            const int *src = reinterpret_cast<const int *>(a.chans + c);
+            int *dst = reinterpret_cast<int *>(copies + i);
+            __syncwarp();
+            for (int w = lane; w < (int)(sizeof(ChannelLaunch) / sizeof(int)); w += 32) dst[w] = src[w];
+            __syncwarp();
+        }
+    }
 };
 
 // Shared memory after the stages: full[S], empty[S], freed[S] (8 bytes
 // each), per stage the consumer warps' sums, the stage headers, and a batch's
-// launch table.
-__host__ __device__ constexpr size_t persist_smem(int stages, size_t stage_bytes, int table = 0)
+// entries in use.
+__host__ __device__ constexpr size_t persist_smem(int stages, size_t stage_bytes, bool batch = false)
 {
     return (size_t)stages * (stage_bytes + 24 + sizeof(StageHeader) + sizeof(double) * NP * kMaxConsumerWarps) +
-           (size_t)table * sizeof(ChannelLaunch);
+           (batch ? (size_t)(stages + kEntries) * sizeof(ChannelLaunch) : 0);
 }
 
 __device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
@@ -405,6 +428,8 @@ __device__ __forceinline__ void flow_loads(const PersistArgs &a, const FlowTable
     unsigned hn = take();
     int c = 0, st = 0, round = 0;
     bool run = true;
+    unsigned citems = chans.entry(0).item_end;  // end of channel c's items
+    chans.fetch(0, 0, lane);
     // the stage `st`, free for new contents
     auto stage_free = [&]() {
         if (round == 0) return true;
@@ -413,9 +438,15 @@ __device__ __forceinline__ void flow_loads(const PersistArgs &a, const FlowTable
     while (run) {
         const unsigned h = __shfl_sync(0xffffffffu, hn, 0);
         hn = take();  // the next item, fetched while this one is waited for and issued
-        while (c < chans.count() && h >= chans[c].item_end) ++c;
-        if (c >= chans.count()) break;
-        const ChannelLaunch &L = chans[c];
+        if (h >= citems) {
+            do {
+                if (++c >= chans.count()) break;
+                citems = chans.entry(c).item_end;
+            } while (h >= citems);
+            if (c >= chans.count()) break;
+            chans.fetch(0, c, lane);
+        }
+        const ChannelLaunch &L = chans.load();
         const ItemPos it = flow_item(h - L.item_first, L.depth, L.lag, L.flow_groups, L.t.gpp, a.nsteps);
         if (it.step < 0) continue;
         const long long abs_step = __ldcg(L.base) + it.step;
@@ -450,6 +481,7 @@ __device__ __forceinline__ void flow_loads(const PersistArgs &a, const FlowTable
         // test switch: the first item is neither armed nor loaded, so its
         // consumers' wait runs out with no copy in flight
         if (!(a.withhold != 0 && h == 0)) {
+            if (!ONE && (round == 0 || sm.hdr[st].chan != c)) chans.fetch(kEntries + st, c, lane);
             if (lane < 3) sm.hdr[st].sh[lane] = sh;
             if (lane < k) sm.hdr[st].rows[lane] = info;
             __syncwarp();
@@ -563,56 +595,57 @@ __device__ __forceinline__ void flow_stores(const PersistArgs &a, const FlowTabl
     volatile int *s_abort = sm.abort;
     // the group whose stores were committed last, not yet announced
     bool pend = false;
-    int pc = 0, pz = 0, pg = 0, pstep = 0;
-    long long pabs = 0;
+    unsigned *pflag = nullptr, *pcount = nullptr, pstep = 0;
     // raise its flag (its copies have landed) and count it in its plane,
     // without waiting for either
     auto announce = [&]() {
-        const ChannelLaunch &L = chans[pc];
         if (lane < Q) fence_async_global();
         __syncwarp();
         if (lane == 0) {
             __threadfence();
-            *reinterpret_cast<volatile unsigned *>(L.flags + (size_t)pz * L.t.gpp + pg) = (unsigned)pstep + 1u;
-            asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(
-                             L.fctr + (size_t)(pabs & (L.p.ring - 1)) * L.p.nz + pz)
-                         : "memory");
+            *reinterpret_cast<volatile unsigned *>(pflag) = pstep + 1u;
+            asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(pcount) : "memory");
         }
     };
     // The plane to look after.  (The warp that counts a plane's last group
     // could sum it instead, but then every count needs its answer, and the sum
     // delays that block's stores: 628x314x200 FP64 7 % slower.)
-    int dc = 0, ds = 0, dz = 0;
-    unsigned dfirst = 0;  // place in the sequence of channel dc's first plane
-    bool dfree = false;   // the counter of the plane is this step's
+    int dc = -1, ds = 0, dz = 0;
+    unsigned dfirst = 0, dn = 0;  // place in the sequence of channel dc's first plane, its (step, plane) pairs
+    bool dfree = false;           // the counter of the plane is this step's
+    long long dabs = 0;
+    const unsigned *dcount = nullptr;
     auto take_duty = [&]() {
         unsigned d = 0;
         if (lane == 0) d = atomicAdd(a.counter + 1, 1u);
         d = __shfl_sync(0xffffffffu, d, 0);
-        for (; dc < chans.count(); ++dc) {
-            const unsigned nz = (unsigned)chans[dc].p.nz, n = nz * (unsigned)a.nsteps;
-            if (d - dfirst < n) {
-                ds = (int)((d - dfirst) / nz);
-                dz = (int)(d - dfirst - (unsigned)ds * nz);
-                break;
-            }
-            dfirst += n;
+        if (d - dfirst >= dn) {
+            do {
+                dfirst += dn;
+                if (++dc >= chans.count()) return;
+                dn = (unsigned)chans.entry(dc).p.nz * (unsigned)a.nsteps;
+            } while (d - dfirst >= dn);
+            chans.fetch(1, dc, lane);
         }
-        dfree = false;
+        const ChannelLaunch &L = chans.duty();
+        ds = (int)((d - dfirst) / (unsigned)L.p.nz);
+        dz = (int)(d - dfirst) - ds * L.p.nz;
+        dabs = __ldcg(L.base) + ds;
+        dcount = L.fctr + (size_t)(dabs & (L.p.ring - 1)) * L.p.nz + dz;
+        dfree = ds < L.p.ring;
     };
     take_duty();
     // true: the plane is done, and the next one taken
     auto service = [&]() {
         if (dc >= chans.count()) return false;
-        const ChannelLaunch &L = chans[dc];
-        const long long abs_step = __ldcg(L.base) + ds;
+        const ChannelLaunch &L = chans.duty();
         if (!dfree) {  // the step that had the counter before has cleared it when it is logged
-            if (!__all_sync(0xffffffffu, ds < L.p.ring || ld_acquire(L.p.step_ctr) > abs_step - L.p.ring)) return false;
+            if (!__all_sync(0xffffffffu, ld_acquire(L.p.step_ctr) > dabs - L.p.ring)) return false;
             dfree = true;
         }
-        const unsigned n = ld_acquire(L.fctr + (size_t)(abs_step & (L.p.ring - 1)) * L.p.nz + dz);
+        const unsigned n = ld_acquire(dcount);
         if (!__all_sync(0xffffffffu, n == (unsigned)L.t.gpp)) return false;
-        flow_plane_done(a, L, abs_step, dz, lane, s_abort);
+        flow_plane_done(a, L, dabs, dz, lane, s_abort);
         take_duty();
         return true;
     };
@@ -661,7 +694,7 @@ __device__ __forceinline__ void flow_stores(const PersistArgs &a, const FlowTabl
             announce();
         }
         const StageHeader &H = sm.hdr[st];
-        const ChannelLaunch &L = chans[H.chan];
+        const ChannelLaunch &L = chans.stage(st);
         const int hc = H.chan, hz = H.z, hg = H.g, hs = H.step;
         const long long habs = H.abs_step;
         unsigned char *stage = sm.stages + (size_t)st * a.stage_bytes;
@@ -676,18 +709,16 @@ __device__ __forceinline__ void flow_stores(const PersistArgs &a, const FlowTabl
             for (int q = lane >> 3; q < nwarps; q += 4) s += w[q * NP];
             s += __shfl_xor_sync(0xffffffffu, s, 8);
             s += __shfl_xor_sync(0xffffffffu, s, 16);
-            const int ring = (int)(habs & (L.p.ring - 1));
-            if (lane < NP) L.fpart[(((size_t)ring * L.p.nz + hz) * L.t.gpp + hg) * NP + lane] = s;
+            const size_t plane = (size_t)(habs & (L.p.ring - 1)) * L.p.nz + hz;
+            if (lane < NP) L.fpart[(plane * L.t.gpp + hg) * NP + lane] = s;
+            pflag = L.flags + (size_t)hz * L.t.gpp + hg;
+            pcount = L.fctr + plane;
+            pstep = (unsigned)hs;
         }
         bulk_wait_read_all();  // the stores have read the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(sm.freed + st);
         pend = true;
-        pc = hc;
-        pz = hz;
-        pg = hg;
-        pstep = hs;
-        pabs = habs;
         if (++st == S) st = 0, par ^= 1u;
         if ((++count & 7u) == 0) service();  // also where the next stage is always ready
     }
@@ -790,7 +821,7 @@ __device__ __forceinline__ void flow_consumers(const PersistArgs &a, const FlowT
         }
         const StageHeader &H = sm.hdr[st];
         if (H.chan < 0) return;
-        const ChannelLaunch &L = chans[H.chan];
+        const ChannelLaunch &L = chans.stage(st);
         const StepArgs &p = L.p;
         const bool q = ANYQ && p.const_q != 0;  // a launch without constant-Q channels compiles no such path
         double G = p.gx;
@@ -865,14 +896,7 @@ __global__ void __launch_bounds__(WIDE ? kTmaMaxThreads : TmaBounds<T, ANYQ>::th
     sm.sums = reinterpret_cast<double *>(sm.freed + S);
     sm.hdr = reinterpret_cast<StageHeader *>(sm.sums + (size_t)S * kMaxConsumerWarps * NP);
     sm.abort = &s_abort;
-    ChannelLaunch *table = reinterpret_cast<ChannelLaunch *>(sm.hdr + S);
-    if constexpr (!ONE) {
-        const int *src = reinterpret_cast<const int *>(a.chans);
-        int *dst = reinterpret_cast<int *>(table);
-        for (int i = threadIdx.x; i < a.nchan * (int)(sizeof(ChannelLaunch) / sizeof(int)); i += blockDim.x)
-            dst[i] = src[i];
-    }
-    const FlowTable<ONE> chans{a, table};
+    const FlowTable<ONE> chans{a, reinterpret_cast<ChannelLaunch *>(sm.hdr + S)};
     if (threadIdx.x == 0) {
         for (int st = 0; st < S; ++st) {
             mbar_init(sm.full + st, 1);

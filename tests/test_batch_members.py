@@ -46,3 +46,27 @@ def test_channel_of_a_batch_stepped_by_itself(prec, mode, monkeypatch):
             np.testing.assert_array_equal(state, want, err_msg=str(spec))
         else:  # sums in another order: the force's rounding, and in FP32 and FP16 the state's
             np.testing.assert_allclose(state, want, rtol=0, atol={64: 1e-11, 32: 1e-5, 16: 1e-3}[prec], err_msg=str(spec))
+
+
+@pytest.mark.parametrize("count,shape,prec", [(10, (720, 3, 4), 64), (3, (740, 3, 4), 64), (60, (628, 3, 4), 64),
+                                              (58, (1256, 3, 4), 32), (450, (8, 4, 3), 64), (2, (2960, 3, 4), 16)])
+def test_number_of_channels_costs_no_shared_memory(count, shape, prec, monkeypatch):
+    """Rows that fill two stages, and many channels: every batch whose widest
+    row fits twice is taken, whatever the number of channels."""
+    monkeypatch.delenv("DNSLBM_BATCH", raising=False)
+    states = [inputs.laminar_state(*shape, 0.05, 0.1, i) for i in range(4)]
+    with dnslbm.Batch([dnslbm.deck(*shape, 1.6, gx=1e-5 * (1 + i % 3), precision=prec) for i in range(count)]) as b:
+        for i, ch in enumerate(b.channels):
+            ch.load_state(states[i % 4])
+        b.step(3)
+        b.step(40)
+        got = [ch.store_state() for ch in b.channels]
+    want = {}
+    for i, state in enumerate(got):
+        key = i % 4, i % 3
+        if key not in want:
+            with dnslbm.Channel(*shape, 1.6, gx=1e-5 * (1 + i % 3), precision=prec) as ch:
+                ch.load_state(states[i % 4])
+                ch.step(43)
+                want[key] = ch.store_state()
+        np.testing.assert_array_equal(state, want[key], err_msg=f"channel {i}")
