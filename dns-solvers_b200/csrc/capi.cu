@@ -559,22 +559,28 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool p
     c->nclean = c->nz;
     c->esize = deck->precision / 8;
     {
-        // rows start on `align` bytes (16 at least, for the bulk copies).
-        // Measured on 628-wide rows: FP32 is faster unpadded (16 bytes: 628,
-        // not 632 elements), FP16 faster on 32 bytes (640, not 632); FP64
-        // rows of 628 are 32-byte multiples either way.
+        // rows start on 16 bytes at least, for the bulk copies (FP64 and FP16
+        // on 32: 628-wide FP16 rows of 640 elements faster than of 632)
         int align_bytes = c->esize == 4 ? 16 : 32;
         const char *e = getenv("DNSLBM_ROW_ALIGN");
         if (e) align_bytes = std::max(16, atoi(e));
         const int v = align_bytes / (int)c->esize;
         c->pitch = (c->nx + v - 1) / v * v;
         if (!c->plain && !e && (size_t)2 * Q * c->pitch * c->esize <= (size_t)216 * 1024) {  // two whole-row stages fit
-            // rows that tensor copies can move in groups of the default size
-            // (tensor_rows): up to 5 % longer
-            size_t row = (size_t)c->pitch * c->esize;
-            const size_t most = row + row / 20;
+            // Longer rows that tensor copies can move (tensor_rows), as long
+            // as a stage still holds three quarters of the rows it did.
+            // Microseconds per step of longer rows / rows as they are: FP64
+            // 628 -> 640 cells 1918 / 1966, 404 -> 416 580 / 734, 204 -> 208
+            // 60.9 / 70.9, 92 -> 96 (7 -> 6 rows) 64.3 / 69.0, but 212 -> 216
+            // (3 -> 2 rows) 164 / 151; FP32 204 -> 208 30.1 / 31.9, 628 -> 640
+            // 927 / 925, but 404 -> 416 244 / 240 (with riblets 260 / 264) and
+            // 644 -> 672 (2 -> 1 rows) 584 / 452: FP32 without solids in the
+            // flow stops at 2 % more bytes, the others at 5 %.
+            const bool tight = c->esize == 4 && deck->bc_mode != DNSLBM_BC_GENERAL;
+            const size_t row0 = (size_t)c->pitch * c->esize, most = row0 + row0 / (tight ? 50 : 20);
+            size_t row = row0;
             while (row <= most && !tensor_rows(row, default_rows(c, row))) row += 16;
-            if (row <= most) c->pitch = (int)(row / c->esize);
+            if (row <= most && 4 * default_rows(c, row) >= 3 * default_rows(c, row0)) c->pitch = (int)(row / c->esize);
         }
     }
     c->ncell = (size_t)c->pitch * c->ny * c->nz;
