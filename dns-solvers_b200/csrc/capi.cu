@@ -185,6 +185,7 @@ struct dnslbm_ctx {
     // channel of nz_all planes, each population array with one ghost plane
     // on either side (pop_off elements from the array's start to plane 0)
     int slab = 0, z0 = 0, nz_all = 0;
+    int member = 0;  // a channel of a batch: its launch shape is the batch's
     int plain = 0;  // rows and groups of the kernels of one launch per step: a slab, ordered_sums, or beside such a channel in a batch
     int wall_lo = 1, wall_hi = 1;
     size_t pop_off = 0;
@@ -2038,7 +2039,8 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
     CK(cudaSetDevice(c->deck.device));
     int ncand = 0;
     double best_ms = 1e30;
-    TmaChoice best = save_choice(c);
+    const TmaChoice own = save_choice(c);
+    TmaChoice best = own;
     int rc;
     // the per-thread kernel
     {
@@ -2127,6 +2129,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
     }
     load_choice(c, best);
     describe_kernel(c);
+    if (c->member) load_choice(c, own);  // the batch's stages and item tables are for its own shape
     // leave the context as created: no state, counters clear
     if ((rc = reset_counters(c))) return rc;
     CK(cudaStreamSynchronize(c->stream));
@@ -2134,6 +2137,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
     if (report && report_len)
         snprintf(report, report_len, "%s: %.4f ms/step (best of %d launch shapes, %d steps each)", c->kernel_desc,
                  best_ms, ncand, steps);
+    if (c->member) describe_kernel(c);
     return DNSLBM_OK;
 }
 
@@ -2527,6 +2531,7 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
             snprintf(g_create_err, sizeof g_create_err, "%s", msg);
             return rc;
         }
+        c->member = 1;
         b->ch.push_back(c);
         if (!c->use_tma) {
             dnslbm_batch_destroy(b);

@@ -294,8 +294,9 @@ int dnslbm_step_timed(dnslbm_ctx *ctx, long nsteps, double *ms_total, double *ms
  * warps) by timing each candidate for `steps` steps on this context's own grid
  * and precision, and keep the fastest.  Call it after dnslbm_create and before
  * a state is set: it steps a rest state and leaves the context without one.
- * report (may be NULL) receives the choice and its time.  No counterpart in
- * the reference, whose loop tiling is the compile-time constant cs
+ * report (may be NULL) receives the choice and its time.  A channel of a
+ * batch keeps the batch's launch shape (dnslbm_batch_autotune chooses it).
+ * No counterpart in the reference, whose loop tiling is the compile-time constant cs
  * (definitions.h:117). */
 int dnslbm_autotune(dnslbm_ctx *ctx, int steps, char *report, size_t report_len);
 

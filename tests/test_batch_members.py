@@ -70,3 +70,28 @@ def test_number_of_channels_costs_no_shared_memory(count, shape, prec, monkeypat
                 ch.step(43)
                 want[key] = ch.store_state()
         np.testing.assert_array_equal(state, want[key], err_msg=f"channel {i}")
+
+
+@pytest.mark.parametrize("mode", ["persistent", "launch"])
+@pytest.mark.parametrize("prec", [64, 16])
+def test_autotune_of_a_batch_channel_leaves_the_batch_its_shape(prec, mode, monkeypatch):
+    """The channel's own search ends with the batch's launch shape: the batch
+    kernel's stages are as large as the batch made them."""
+    monkeypatch.setenv("DNSLBM_BATCH", mode)
+    chans = [_make(s, prec) for s in (SPECS[0], SPECS[2], SPECS[4])]
+    with dnslbm.Batch([dnslbm.deck(*shape, 1.7, **kw) for shape, _, _, kw in chans]) as b:
+        kernel = b.kernel
+        for ch in b.channels:
+            assert "best of" in ch.autotune(2)
+        assert b.kernel == kernel
+        for ch, (_, fl, st, _) in zip(b.channels, chans):
+            ch.set_flags(fl)
+            ch.load_state(st)
+        b.step(38)
+        got = [ch.store_state() for ch in b.channels]
+    for (shape, fl, st, kw), state in zip(chans, got):
+        with dnslbm.Channel(*shape, 1.7, **kw) as ch:
+            ch.set_flags(fl)
+            ch.load_state(st)
+            ch.step(38)
+            np.testing.assert_array_equal(state, ch.store_state())
