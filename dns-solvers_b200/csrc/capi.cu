@@ -514,10 +514,38 @@ static int step_consumers(const dnslbm_ctx *c)
     return std::min(cap, (c->nx + 31) / 32 * 32);
 }
 
+// The memory the persistent kernel needs for the row groups of the channel's
+// launch shape: taken when the shape is chosen, never by a step.  What was
+// there stays if more cannot be had.
+static int flow_reserve(dnslbm_ctx *c)
+{
+    const size_t groups = (size_t)c->tma.gpp * c->nz, part = (size_t)kRing * groups * NP;
+    auto grow = [&](void **p, size_t &have, size_t want, size_t size) {
+        if (want <= have) return true;
+        void *q = nullptr;
+        if (cudaMalloc(&q, want * size) != cudaSuccess) {
+            cudaGetLastError();
+            fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", want * size);
+            return false;
+        }
+        if (*p) cudaFree(*p);
+        *p = q;
+        have = want;
+        return true;
+    };
+    if (!grow((void **)&c->flow_flags, c->flow_flags_n, groups, sizeof(unsigned)) ||
+        !grow((void **)&c->flow_part, c->flow_part_n, part, sizeof(double)))
+        return DNSLBM_ERR_NOMEM;
+    return DNSLBM_OK;
+}
+
+// Rows of a channel's arrays: made longer for tensor copies where that pays,
+// never, or (plain) as for a channel with ordered sums.
+enum Rows { kRowsAny, kRowsShort, kRowsPlain };
+
 // A whole channel (slab = 0) or the wall-normal slab [z0, z0 + nzs) of one
 // (slab = 1, dnslbm_create_slab).
-// plain: rows as for a channel with ordered sums.
-static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool plain, dnslbm_ctx **out)
+static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, Rows rows, dnslbm_ctx **out)
 {
     dnslbm_ctx *c = nullptr;
     if (!deck || !out) return fail(c, DNSLBM_ERR_ARG, "null deck or output pointer");
@@ -552,7 +580,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool p
     c->ny = deck->ydv;
     c->nz = slab ? nzs : deck->zdv;
     c->slab = slab;
-    c->plain = slab || plain || ordered_sums(*deck);
+    c->plain = slab || rows == kRowsPlain || ordered_sums(*deck);
     c->z0 = slab ? z0 : 0;
     c->nz_all = deck->zdv;
     c->wall_lo = c->z0 == 0;
@@ -567,7 +595,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool p
         if (e) align_bytes = std::max(16, atoi(e));
         const int v = align_bytes / (int)c->esize;
         c->pitch = (c->nx + v - 1) / v * v;
-        if (!c->plain && !e && (size_t)2 * Q * c->pitch * c->esize <= (size_t)216 * 1024) {  // two whole-row stages fit
+        if (!c->plain && rows == kRowsAny && !e && (size_t)2 * Q * c->pitch * c->esize <= (size_t)216 * 1024) {  // two whole-row stages fit
             // Longer rows that tensor copies can move (tensor_rows), as long
             // as a stage still holds three quarters of the rows it did.
             // Microseconds per step of longer rows / rows as they are: FP64
@@ -689,6 +717,7 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool p
         }
         cudaMemset(*a.p, 0, a.bytes);
     }
+    if (uses_flow(c) && flow_reserve(c)) return bail(DNSLBM_ERR_NOMEM);
     if (slab) {
         const size_t bytes = (size_t)2 * c->nz_all * 3 * sizeof(double);
         if (cudaMalloc((void **)&c->shift_all, bytes) != cudaSuccess) {
@@ -726,11 +755,22 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, bool p
     return DNSLBM_OK;
 }
 
-extern "C" int dnslbm_create(const dnslbm_deck *deck, dnslbm_ctx **out) { return create_ctx(deck, 0, 0, 0, false, out); }
+// Where longer rows do not fit the device's memory, rows as they are may.
+static int create_channel(const dnslbm_deck *deck, Rows rows, dnslbm_ctx **out)
+{
+    int rc = create_ctx(deck, 0, 0, 0, rows, out);
+    if (rc == DNSLBM_ERR_NOMEM && rows == kRowsAny) {
+        cudaGetLastError();
+        rc = create_ctx(deck, 0, 0, 0, kRowsShort, out);
+    }
+    return rc;
+}
+
+extern "C" int dnslbm_create(const dnslbm_deck *deck, dnslbm_ctx **out) { return create_channel(deck, kRowsAny, out); }
 
 extern "C" int dnslbm_create_slab(const dnslbm_deck *deck, int z0, int nzs, dnslbm_ctx **out)
 {
-    return create_ctx(deck, 1, z0, nzs, false, out);
+    return create_ctx(deck, 1, z0, nzs, kRowsPlain, out);
 }
 
 extern "C" void dnslbm_destroy(dnslbm_ctx *c)
@@ -1116,33 +1156,6 @@ extern "C" int dnslbm_store_state(dnslbm_ctx *c, double *state)
                            cudaMemcpyDeviceToHost, c->stream));
     }
     CK(cudaStreamSynchronize(c->stream));
-    return DNSLBM_OK;
-}
-
-// The memory the persistent kernel needs for the channel's row groups.
-static int flow_reserve(dnslbm_ctx *c)
-{
-    const size_t groups = (size_t)c->tma.gpp * c->nz, part = (size_t)kRing * groups * NP;
-    if (groups > c->flow_flags_n) {
-        if (c->flow_flags) CK(cudaFree(c->flow_flags));
-        c->flow_flags = nullptr;
-        c->flow_flags_n = 0;
-        if (cudaMalloc((void **)&c->flow_flags, groups * sizeof(unsigned)) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", groups * sizeof(unsigned));
-        }
-        c->flow_flags_n = groups;
-    }
-    if (part > c->flow_part_n) {
-        if (c->flow_part) CK(cudaFree(c->flow_part));
-        c->flow_part = nullptr;
-        c->flow_part_n = 0;
-        if (cudaMalloc((void **)&c->flow_part, part * sizeof(double)) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", part * sizeof(double));
-        }
-        c->flow_part_n = part;
-    }
     return DNSLBM_OK;
 }
 
@@ -2072,6 +2085,9 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
         if (ms < bt.ms) bt.ms = ms, bt.ch = save_choice(c), bt.k = k, bt.st = st, bt.seg = seg, bt.cons = cons;
         return DNSLBM_OK;
     };
+    auto configure = [&](int k, int st, int cons, int bps, int seg) {
+        return tma_configure(c, k, st, cons, bps, seg) || (uses_flow(c) && flow_reserve(c));
+    };
     // the default consumer count and the widest consumer sets (a block with
     // large stages is alone on its SM and needs more warps)
     const int widest = std::min(352, (c->nx + 31) / 32 * 32 + 32);
@@ -2079,7 +2095,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
         for (int st : {2, 3, 4})
             for (int cons : {cons0, 224, widest}) {
                 if ((cons != cons0 && (cons <= cons0 || (cons == 224 && widest <= 224))) || k > c->ny ||
-                    tma_configure(c, k, st, cons, 0))
+                    configure(k, st, cons, 0, 0))
                     continue;
                 if ((rc = timed(k, st, 0, cons))) return rc;
             }
@@ -2089,7 +2105,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
         for (int nseg : {2, 3, 4})
             for (int st : {2, 3, 4}) {
                 const int seg = segment_for(c->nx, nseg);
-                if (tma_configure(c, 1, st, cons0, 0, seg)) continue;
+                if (configure(1, st, cons0, 0, seg)) continue;
                 if ((rc = timed(1, st, seg, cons0))) return rc;
             }
     // consumer counts, then a cap on the blocks per SM, for each parity's best
@@ -2101,7 +2117,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
             seen |= leaders[q].k == b0.k && leaders[q].st == b0.st && leaders[q].seg == b0.seg;
         if (b0.k < 0 || seen) continue;
         for (int cons = 64; cons <= widest; cons += 32) {
-            if (cons == cons0 || cons == 224 || cons == widest || tma_configure(c, b0.k, b0.st, cons, 0, b0.seg)) continue;
+            if (cons == cons0 || cons == 224 || cons == widest || configure(b0.k, b0.st, cons, 0, b0.seg)) continue;
             if ((rc = timed(b0.k, b0.st, b0.seg, cons))) return rc;
         }
     }
@@ -2110,7 +2126,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
         const Best b0 = leaders2[pass];
         if (b0.k < 0) continue;
         for (int bps : {1, 2, 3}) {
-            if (tma_configure(c, b0.k, b0.st, b0.cons, bps, b0.seg)) continue;
+            if (configure(b0.k, b0.st, b0.cons, bps, b0.seg)) continue;
             if ((rc = timed(b0.k, b0.st, b0.seg, b0.cons))) return rc;
         }
     }
@@ -2161,6 +2177,7 @@ struct dnslbm_batch {
     int pgrid = 0;                      // its blocks
     size_t pstage = 0, psmem = 0;       // bytes of one stage, dynamic shared memory
     int general = 0;                    // some channel may have planes with link masks
+    int nomem = 0;                      // the last shape tried asked for more memory than there is
     int any_links = 0;                  // some channel has planes with link masks
     ChannelLaunch *d_flow = nullptr;    // [2][n] the launch tables of a full chunk and of what is left of a call
     std::vector<ChannelLaunch> flow_host[2];  // what d_flow holds
@@ -2432,6 +2449,7 @@ static int member_shape(dnslbm_ctx *c, int stages, int consumers)
 static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consumers)
 {
     const bool flow = b->flow();
+    b->nomem = 0;
     const int special = flow ? 64 : 32;  // threads of the load and store warps, or of the producer
     consumers = std::max(32, std::min(flow ? 32 * kMaxConsumerWarps : 352, consumers / 32 * 32));
     size_t smem = 0;
@@ -2501,6 +2519,11 @@ static int batch_configure(dnslbm_batch *b, size_t budget, int stages, int consu
                 return -1;
         }
     }
+    for (auto *c : b->ch)
+        if (uses_flow(c) && flow_reserve(c)) {
+            b->nomem = 1;
+            return -1;
+        }
     destroy_graphs(b);
     batch_layout(b);
     return 0;
@@ -2523,7 +2546,7 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
     for (int i = 0; i < n; ++i) b->ordered |= ordered_sums(decks[i]);
     for (int i = 0; i < n; ++i) {
         dnslbm_ctx *c = nullptr;
-        int rc = create_ctx(&decks[i], 0, 0, 0, b->ordered != 0, &c);
+        int rc = create_channel(&decks[i], b->ordered ? kRowsPlain : kRowsAny, &c);
         if (rc) {
             char msg[512];
             snprintf(msg, sizeof msg, "channel %d: %s", i, g_create_err);
@@ -2557,7 +2580,8 @@ extern "C" int dnslbm_batch_create(const dnslbm_deck *decks, int n, dnslbm_batch
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     if (batch_configure(b, budgets[!b->flow()], 2, consumers) && batch_configure(b, budgets[b->flow()], 2, consumers) &&
         (!b->flow() || batch_configure(b, (size_t)maxsmem - kPersistSmemReserve, 2, consumers)))
-        return bail(bfail(b, DNSLBM_ERR_ARG, "batched kernel does not fit the device"));
+        return bail(b->nomem ? bfail(b, DNSLBM_ERR_NOMEM, "not enough device memory for the batch's row groups")
+                             : bfail(b, DNSLBM_ERR_ARG, "batched kernel does not fit the device"));
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev[0]) != cudaSuccess || cudaEventCreate(&b->ev[1]) != cudaSuccess ||
         cudaMalloc(&b->d_launch, sizeof(ChannelLaunch) * n) != cudaSuccess ||
