@@ -157,7 +157,7 @@ struct dnslbm_ctx {
     cudaEvent_t out_ev[2] = {nullptr, nullptr};
     int out_pending = 0;
     double *quad_buf = nullptr;  // quadrant analysis: plane means [zd][3], plane sums [zd][9]
-    double *post_ws = nullptr;   // scratch and results of the post-processing calls, kept between calls
+    double *post_ws = nullptr;   // scratch and results of the post-processing calls, see post_workspace
     size_t post_ws_n = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> tev;  // per-launch timing events
@@ -1718,21 +1718,25 @@ static void quadrant_finish(int zd, double n, const double *sums, double *quadra
     }
 }
 
-// At least n doubles of the context's post-processing workspace.
-static int post_reserve(dnslbm_ctx *c, size_t n)
+// The context's post-processing workspace, n doubles of it; nullptr where the
+// call is to use memory of its own: a workspace of more than kPostKeep bytes
+// (628x314x200 spectra want 0.95 GB) is not kept from call to call, and what
+// cannot be had for keeping may do for the call's time.
+constexpr size_t kPostKeep = (size_t)512 << 20;
+static double *post_workspace(dnslbm_ctx *c, size_t n)
 {
-    if (n <= c->post_ws_n) return DNSLBM_OK;
-    if (c->post_ws) CK(cudaFree(c->post_ws));
+    if (n * sizeof(double) > kPostKeep) return nullptr;
+    if (n <= c->post_ws_n) return c->post_ws;
+    if (c->post_ws) cudaFree(c->post_ws);
     c->post_ws = nullptr;
     c->post_ws_n = 0;
-    const cudaError_t e = cudaMalloc((void **)&c->post_ws, n * sizeof(double));
-    if (e != cudaSuccess) {
+    if (cudaMalloc((void **)&c->post_ws, n * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
-        return fail(c, DNSLBM_ERR_NOMEM, "cudaMalloc of %zu bytes of post-processing workspace failed: %s",
-                    n * sizeof(double), cudaGetErrorString(e));
+        c->post_ws = nullptr;
+        return nullptr;
     }
     c->post_ws_n = n;
-    return DNSLBM_OK;
+    return c->post_ws;
 }
 
 extern "C" int dnslbm_quadrant(dnslbm_ctx *c, double *quadrant, double *dquadrant, double *uw)
@@ -1750,9 +1754,12 @@ extern "C" int dnslbm_quadrant(dnslbm_ctx *c, double *quadrant, double *dquadran
     // the velocity field in the vel layout, then the two plane passes
     if (c->out_pending) CK(cudaStreamWaitEvent(c->stream, c->out_ev[1], 0));
     launch_io(c->deck.precision, 3, io_args(c), 0, c->nx, c->out_vel, c->out_den, c->stream);
-    if ((rc = post_reserve(c, quadrant_scratch(c->nx, c->ny, zd)))) return rc;
-    launch_quadrant(c->out_vel, c->nx, c->ny, zd, c->post_ws, c->quad_buf, c->quad_buf + (size_t)zd * 3, c->stream);
-    CK(cudaGetLastError());
+    double *ws = post_workspace(c, quadrant_scratch(c->nx, c->ny, zd)), *own = nullptr;
+    if (!ws) CK(cudaMalloc((void **)&own, quadrant_scratch(c->nx, c->ny, zd) * sizeof(double)));
+    launch_quadrant(c->out_vel, c->nx, c->ny, zd, ws ? ws : own, c->quad_buf, c->quad_buf + (size_t)zd * 3, c->stream);
+    const cudaError_t launched = cudaGetLastError();
+    if (own) cudaFree(own);  // after the kernels that use it
+    CK(launched);
     std::vector<double> sums((size_t)zd * 9);
     CK(cudaMemcpyAsync(sums.data(), c->quad_buf + (size_t)zd * 3, sums.size() * sizeof(double), cudaMemcpyDeviceToHost,
                        c->stream));
@@ -1833,8 +1840,8 @@ extern "C" int dnslbm_correlations(dnslbm_ctx *c, double *xcorl, double *ycorl, 
     if (c->out_pending) CK(cudaStreamWaitEvent(c->stream, c->out_ev[1], 0));
     launch_io(c->deck.precision, 3, io_args(c), 0, c->nx, c->out_vel, c->out_den, c->stream);
     CK(cudaGetLastError());
-    if ((rc = post_reserve(c, correlations_ws(c->nx, c->ny, zd)))) return rc;
-    const cudaError_t e = correlations_of(c->out_vel, c->nx, c->ny, zd, c->stream, c->post_ws, xcorl, ycorl, uavg);
+    double *ws = post_workspace(c, correlations_ws(c->nx, c->ny, zd));
+    const cudaError_t e = correlations_of(c->out_vel, c->nx, c->ny, zd, c->stream, ws, xcorl, ycorl, uavg);
     if (e != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "correlations: %s", cudaGetErrorString(e));
     return DNSLBM_OK;
 }
@@ -1908,8 +1915,8 @@ extern "C" int dnslbm_spectra(dnslbm_ctx *c, double *ex, double *ey)
     if (c->out_pending) CK(cudaStreamWaitEvent(c->stream, c->out_ev[1], 0));
     launch_io(c->deck.precision, 3, io_args(c), 0, c->nx, c->out_vel, c->out_den, c->stream);
     CK(cudaGetLastError());
-    if ((rc = post_reserve(c, spectra_ws(c->nx, c->ny, zd)))) return rc;
-    const cudaError_t e = spectra_of(c->out_vel, c->nx, c->ny, zd, c->stream, c->post_ws, ex, ey);
+    double *ws = post_workspace(c, spectra_ws(c->nx, c->ny, zd));
+    const cudaError_t e = spectra_of(c->out_vel, c->nx, c->ny, zd, c->stream, ws, ex, ey);
     if (e != cudaSuccess) return fail(c, DNSLBM_ERR_CUDA, "spectra: %s", cudaGetErrorString(e));
     return DNSLBM_OK;
 }

@@ -275,9 +275,9 @@ int dnslbm_correlations_vel(const double *vel, int xdv, int ydv, int zdv, int de
  *   ey[3][ydv/2+1][zd]   Euuy, Evvy, Ewwy (per spanwise mode j),
  * the program's file layouts ([mode][zd] per component, wall planes 0).  The
  * transforms are evaluated directly in FP64 (the program calls FFTW), to
- * rounding of the DFT.  The workspace of the context's post-processing calls
- * (here about 0.7 times 16 bytes per velocity value) is kept until
- * dnslbm_destroy.  Either pointer may be NULL. */
+ * rounding of the DFT.  A context keeps a workspace of its post-processing
+ * calls of up to 512 MB; a call that needs more (here about 0.7 times 16 bytes
+ * per velocity value) takes and returns it.  Either pointer may be NULL. */
 int dnslbm_spectra(dnslbm_ctx *ctx, double *ex, double *ey);
 /* The same for a velocity field read from a vel.NNNN file
  * ([xdv][ydv][zdv+2][3] doubles), on CUDA device `device`. */

@@ -56,3 +56,18 @@ def test_longer_rows_give_way_to_memory():
     finally:
         chunks.clear()
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("shape,kept", [((400, 400, 140), False), ((200, 60, 40), True)])
+def test_large_workspaces_are_given_back(shape, kept):
+    """Spectra's workspace is about nx * ny / 2 * nz * 48 bytes; above 512 MB
+    it lives for the call."""
+    with dnslbm.Channel(*shape, 1.6, gx=1e-5, precision=16) as ch:
+        ch.init_rest()
+        ch.quadrant()  # takes the velocity field's memory
+        before = _free()
+        ch.spectra()
+        after = _free()
+        assert before - after <= (512 << 20 if kept else 0)
+        ch.spectra()
+        assert _free() == after
