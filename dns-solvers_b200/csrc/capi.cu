@@ -2193,6 +2193,7 @@ struct dnslbm_batch {
     unsigned groups = 0;                // row groups of all channels
     unsigned *d_counter = nullptr;      // items and planes taken
     int *d_abort = nullptr;             // a bounded wait of the launch gave up
+    unsigned long long graph_wait_ns = 0;  // the wait limit the graphs were captured with
     int graph_ok = 1;                   // 0: stream capture of the launch was refused
     int withhold = 0;                   // test hook: the next run withholds a load
     unsigned long long withhold_wait_ns = 0;
@@ -2743,6 +2744,8 @@ static int persist_run(dnslbm_batch *b, long nsteps)
     for (auto *c : b->ch) groups += (double)c->tma.gpp * c->nz;
     const int chunk = b->flow() ? std::min(b->graph_steps, flow_chunk(groups)) : b->graph_steps;
     int odd = b->ch[0]->odd;
+    if (b->graph_wait_ns != b->ch[0]->wait_ns) destroy_graphs(b);
+    b->graph_wait_ns = b->ch[0]->wait_ns;
     while (left > 0) {
         const int n = (int)std::min<long>(left, chunk), slot = n == chunk ? 0 : 1;
         if (b->flow())

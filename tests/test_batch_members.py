@@ -95,3 +95,29 @@ def test_autotune_of_a_batch_channel_leaves_the_batch_its_shape(prec, mode, monk
             ch.load_state(st)
             ch.step(38)
             np.testing.assert_array_equal(state, ch.store_state())
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_wait_limit_set_after_a_chunk_of_steps(prec, monkeypatch):
+    """The limit of channel 0 holds for the chunks replayed from a graph too: a
+    limit shorter than any load ends the next chunk, and the states can be
+    loaded again."""
+    monkeypatch.delenv("DNSLBM_BATCH", raising=False)
+    chans = [_make(s, prec) for s in SPECS[:2]]
+    with dnslbm.Batch([dnslbm.deck(*shape, 1.7, **kw) for shape, _, _, kw in chans]) as b:
+        def load():
+            for ch, (_, fl, st, _) in zip(b.channels, chans):
+                ch.set_flags(fl)
+                ch.load_state(st)
+        load()
+        b.step(64)
+        want = [ch.store_state() for ch in b.channels]
+        b.channels[0].set_wait_limit(1e-5)
+        with pytest.raises(dnslbm.DnsLbmError) as e:
+            b.step(64)
+        assert e.value.code == dnslbm.ERR_TIMEOUT
+        b.channels[0].set_wait_limit(1000)
+        load()
+        b.step(64)
+        for ch, w in zip(b.channels, want):
+            np.testing.assert_array_equal(ch.store_state(), w)
