@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import dnslbm
+import inputs
 
 pytestmark = pytest.mark.gpu
 SHAPES = [(1, 1, 1), (2, 3, 1), (7, 8, 2), (16, 17, 5), (31, 64, 6), (67, 40, 9), (2048, 3, 1), (5, 1500, 2)]
@@ -65,3 +66,26 @@ def test_quadrants(shape):
     for i, s in enumerate(((u > 0) & (w > 0), (u < 0) & (w > 0), (u < 0) & (w < 0), (u > 0) & (w < 0))):
         _close(dq[i, 1:-1], (u * w * s).sum((0, 1)) / (nx * ny))
     _close(uw[1:-1], (u * w).sum((0, 1)) / (nx * ny))
+
+
+@pytest.mark.parametrize("prec", [64, 32, 16])
+@pytest.mark.parametrize("shape", [(33, 5, 6), (32, 3, 14), (2, 2, 3), (70, 4, 9)])
+def test_moments_of_a_state(shape, prec):
+    """Tiles of 32 x 8 planes (walls included) of one y: edges of both.  The
+    fields against the stored populations: 19 FP64 additions in the same order
+    and one division, up to the stored values' own rounding (none here: they
+    are read back from the same state); wall planes are zero."""
+    nx, ny, nz = shape
+    with dnslbm.Channel(nx, ny, nz, 1.7, gx=2e-5, precision=prec) as ch:
+        ch.load_state(inputs.laminar_state(nx, ny, nz, 0.06, 0.1, 3))
+        for steps in (0, 1, 1):
+            ch.step(steps)
+            f = ch.store_state()
+            vel, den = ch.moments()
+            e = np.asarray(inputs.E, float)
+            rho = f.sum(-1)
+            np.testing.assert_allclose(den, rho, rtol=0, atol=1e-14)
+            j = f @ e
+            j[:, :, 1:-1] /= rho[:, :, 1:-1, None]
+            np.testing.assert_allclose(vel, j, rtol=0, atol=1e-14)
+            assert not vel[:, :, [0, -1]].any() and not den[:, :, [0, -1]].any()
