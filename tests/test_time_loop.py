@@ -62,3 +62,45 @@ def test_planes_with_link_masks(prec, walls, monkeypatch):
     if walls != "riblets":  # a block in the flow: rows of solid and fluid cells
         flags[5:11, 8:15, 5:9] = -1
     _compare(shape, flags, prec, (1, 9), monkeypatch, general=True)
+
+
+def _beyond_l2(texture, prec):
+    """A grid whose state does not stay in L2; FP32 rows of 402 cells are 1616
+    bytes, three to a group, which tensor copies cannot take."""
+    shape = {64: (301, 57, 44), 32: (402, 75, 52), 16: (640, 83, 60)}[prec]
+    if texture == "grooves":
+        return shape, inputs.flags_longitudinal(*shape, 3, 5), False
+    flags = inputs.flags_riblets(*shape, 3, 6)  # rows alike, and a block in the flow: mixed rows
+    flags[5:11, 8:15, 20:24] = -1
+    return shape, flags, True
+
+
+@pytest.mark.parametrize("prec", [64, 32, 16])
+@pytest.mark.parametrize("texture", ["grooves", "riblets and a block"])
+def test_two_steps_at_once_with_wall_links(texture, prec, monkeypatch):
+    """Results written by the threads themselves (links of a textured wall, of
+    mixed rows) and read by another step's copies two steps deep, over calls of
+    odd and even lengths."""
+    shape, flags, general = _beyond_l2(texture, prec)
+    kernel = _compare(shape, flags, prec, (3, 70, 1), monkeypatch, general)
+    assert "2 steps per sweep" in kernel, kernel
+
+
+def test_two_steps_at_once_in_a_batch(monkeypatch):
+    """A channel two steps deep between channels of one step at a time."""
+    monkeypatch.delenv("DNSLBM_BATCH", raising=False)
+    shape, flags, general = _beyond_l2("riblets and a block", 32)
+    small = 45, 17, 5
+    specs = [(small, inputs.flags_longitudinal(*small, 1, 1), False), (shape, flags, general), (small, inputs.flags_smooth(*small), False)]
+    decks = [dnslbm.deck(*s, 1.7, gx=2e-5, precision=32, bc_mode=dnslbm.BC_GENERAL if g else dnslbm.BC_REFERENCE)
+             for s, _, g in specs]
+    with dnslbm.Batch(decks) as b:
+        for ch, (s, fl, _) in zip(b.channels, specs):
+            ch.set_flags(fl)
+            ch.load_state(inputs.laminar_state(*s, 0.06, 0.1, 7))
+        for n in (3, 70, 1):
+            b.step(n)
+        got = [ch.store_state() for ch in b.channels]
+    for (s, fl, g), state in zip(specs, got):
+        _, want, _ = _run("scalar", s, fl, 32, (3, 70, 1), g, monkeypatch)
+        np.testing.assert_array_equal(state, want)
