@@ -59,6 +59,11 @@ struct StepArgs {
     // of the state before it), else a power of two R for [R][nz][3] (step s
     // reads the means of state s - R, or of the loaded state)
     int ring = 0;
+    // FP32 and FP16 whole channels: the force of a constant flow rate by a
+    // fused multiply-add.  A step with solids in the flow has two kernels,
+    // either of which may run the tail, and the compiler fuses the product in
+    // one of them only: the force's last bits depended on which came last.
+    int fused_force = 0;
 };
 
 // The shift c(z) of a step's energy sum: the plane means entry it reads.
@@ -294,7 +299,8 @@ __device__ __forceinline__ void tail_planes(const StepArgs &a, long long step, i
 __device__ __forceinline__ double tail_force(const StepArgs &a, double rho, double jx)
 {
     const double N = (double)a.nx * (double)a.ny * (double)a.nz;
-    return a.const_q ? (rho / N) * a.ubulk - jx / N : a.gx;
+    if (!a.const_q) return a.gx;
+    return a.fused_force ? fma(rho / N, a.ubulk, -(jx / N)) : (rho / N) * a.ubulk - jx / N;
 }
 
 // force: also set the next step's force.
