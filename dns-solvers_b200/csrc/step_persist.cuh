@@ -179,6 +179,18 @@ struct FlowTable {
         if constexpr (ONE) return a.one_maps;
         else return a.maps[c];
     }
+    // Before the block's first use of channel c's tensor maps, which the host
+    // has written to global memory (and may write anew between launches).
+    __device__ __forceinline__ void fence_maps(int c, int lane) const
+    {
+        if constexpr (!ONE) {
+            if (lane < (int)(sizeof(FlowMaps) / sizeof(CUtensorMap)))
+                asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(
+                                 reinterpret_cast<const CUtensorMap *>(a.maps + c) + lane)
+                             : "memory");
+            __syncwarp();
+        }
+    }
     // copy i of entry c, by the whole warp that uses it
     __device__ __forceinline__ void fetch(int i, int c, int lane) const
     {
@@ -430,6 +442,7 @@ __device__ __forceinline__ void flow_loads(const PersistArgs &a, const FlowTable
     bool run = true;
     unsigned citems = chans.entry(0).item_end;  // end of channel c's items
     chans.fetch(0, 0, lane);
+    chans.fence_maps(0, lane);  // the store warp's uses follow the load warp's through the stage's barriers
     // the stage `st`, free for new contents
     auto stage_free = [&]() {
         if (round == 0) return true;
@@ -445,6 +458,7 @@ __device__ __forceinline__ void flow_loads(const PersistArgs &a, const FlowTable
             } while (h >= citems);
             if (c >= chans.count()) break;
             chans.fetch(0, c, lane);
+            chans.fence_maps(c, lane);
         }
         const ChannelLaunch &L = chans.load();
         const ItemPos it = flow_item(h - L.item_first, L.depth, L.lag, L.flow_groups, L.t.gpp, a.nsteps);
