@@ -269,7 +269,6 @@ static StepArgs step_args(const dnslbm_ctx *c)
     p.wall_hi = c->wall_hi;
     p.tail = c->slab ? 0 : 1;
     p.ring = uses_flow(c) ? kRing : 0;
-    p.fused_force = !c->slab && c->deck.precision != 64;
     return p;
 }
 

@@ -300,7 +300,7 @@ __device__ __forceinline__ void persist_consumers(const PersistArgs &a, int s, u
         const bool done = H.group == H.it.count - 1;
         if (done) {  // the item is done: its plane contribution (the stage is released after it)
             // step -1: the channel's step tail reads its own step counter
-            plane_contribute(p, acc, z, H.it.slot, H.it.ncontrib, -1, G, 0, nc);
+            plane_contribute<true, true>(p, acc, z, H.it.slot, H.it.ncontrib, -1, G, 0, nc);
 #pragma unroll
             for (int r = 0; r < NP; ++r) acc[r] = 0.0;
         }

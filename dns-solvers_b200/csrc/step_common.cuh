@@ -59,20 +59,19 @@ struct StepArgs {
     // of the state before it), else a power of two R for [R][nz][3] (step s
     // reads the means of state s - R, or of the loaded state)
     int ring = 0;
-    // FP32 and FP16 whole channels: the force of a constant flow rate by a
-    // fused multiply-add.  A step with solids in the flow has two kernels,
-    // either of which may run the tail, and the compiler fuses the product in
-    // one of them only: the force's last bits depended on which came last.
-    int fused_force = 0;
 };
 
 // The shift c(z) of a step's energy sum: the plane means entry it reads.
 // Any recent means serve (the shift only keeps the one-pass variance free of
 // cancellation).  A ring lets steps overlap: step s needs no sums of the
-// steps just before it.
+// steps just before it.  RING false: the per-thread FP64 kernel, whose
+// contexts have none and which is 6 % slower over a whole grid if its code so
+// much as asks (402x201x64 350 us per step, 372 with the question; the other
+// kernels are no slower for it).
+template <bool RING = true>
 __device__ __forceinline__ const double *shift_entry(const StepArgs &p, long long step)
 {
-    return p.shift + (size_t)(step & (p.ring ? p.ring - 1 : 1)) * p.nz * 3;
+    return p.shift + (size_t)(step & (RING && p.ring ? p.ring - 1 : 1)) * p.nz * 3;
 }
 
 // -1: plane z lies next to the bottom wall, +1: next to the top wall, 0:
@@ -263,13 +262,15 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *smem)
 // Two parts, shared by the block-wide tail below and the persistent
 // kernel's one-warp tail: the sums over the planes (this thread's planes z0,
 // z0 + stride, ...), and the record of the summed totals.
+template <bool RING = true>
 __device__ __forceinline__ void tail_planes(const StepArgs &a, long long step, int mode, const double *plane_sums, int z0,
                                             int stride, double (&t)[6])
 {
     const int nz = a.nz;
     const double np = (double)a.nx * (double)a.ny;
-    const double *cshift = shift_entry(a, step);
-    double *nshift = const_cast<double *>(a.ring || mode != 0 ? shift_entry(a, step) : shift_entry(a, step + 1));
+    const bool ring = RING && a.ring;
+    const double *cshift = shift_entry<RING>(a, step);
+    double *nshift = const_cast<double *>(shift_entry<RING>(a, ring || mode != 0 ? step : step + 1));
     for (int z = z0; z < nz; z += stride) {
         const double *ps = plane_sums + (size_t)z * NP;
         double s[NP];
@@ -285,7 +286,7 @@ __device__ __forceinline__ void tail_planes(const StepArgs &a, long long step, i
         t[4] += s[6];
         t[5] += s[7];
         // a loaded state fills every entry of a ring
-        const int copies = a.ring && mode != 0 ? a.ring : 1;
+        const int copies = ring && mode != 0 ? a.ring : 1;
         for (int r = 0; r < copies; ++r) {
             double *n = copies > 1 ? a.shift + (size_t)r * nz * 3 : nshift;
             n[z * 3 + 0] = um;
@@ -296,14 +297,20 @@ __device__ __forceinline__ void tail_planes(const StepArgs &a, long long step, i
 }
 
 // The force of the next step from the writer-side totals (encalc.c:121).
+// FUSED (FP32 and FP16 whole channels): by a fused multiply-add.  A step with
+// solids in the flow has two kernels, either of which may run the tail, and
+// left to itself the compiler fuses the product in one of them only: the
+// force's last bits would depend on which came last.
+template <bool FUSED>
 __device__ __forceinline__ double tail_force(const StepArgs &a, double rho, double jx)
 {
     const double N = (double)a.nx * (double)a.ny * (double)a.nz;
     if (!a.const_q) return a.gx;
-    return a.fused_force ? fma(rho / N, a.ubulk, -(jx / N)) : (rho / N) * a.ubulk - jx / N;
+    return FUSED ? fma(rho / N, a.ubulk, -(jx / N)) : (rho / N) * a.ubulk - jx / N;
 }
 
 // force: also set the next step's force.
+template <bool FUSED>
 __device__ __forceinline__ void tail_record(const StepArgs &a, long long step, double force_used, int mode,
                                             const double *plane_sums, const double (&t)[6], bool force = true)
 {
@@ -338,18 +345,19 @@ __device__ __forceinline__ void tail_record(const StepArgs &a, long long step, d
     if (stress != stress && __ldcg(a.status) == 0) a.status[0] = step + 1;
     // constant-Q: next force from the totals of the state this step wrote
     // (encalc.c:121 evaluated one step ahead); sum of populations = t[4]
-    if (force) a.force[(step + 1) & 1] = tail_force(a, t[4], t[5]);
+    if (force) a.force[(step + 1) & 1] = tail_force<FUSED>(a, t[4], t[5]);
 }
 
+template <bool RING, bool FUSED>
 static __device__ __forceinline__ void step_tail(const StepArgs &a, long long step, double force_used, int mode, double *smem,
                                                  int nthreads)
 {
     if (step < 0) step = __ldcg(a.step_ctr);
     double t[6] = {0, 0, 0, 0, 0, 0};  // rho, jx, sum of plane means u, K, writer rho, writer jx
-    tail_planes(a, step, mode, a.plane_sums, threadIdx.x, nthreads, t);
+    tail_planes<RING>(a, step, mode, a.plane_sums, threadIdx.x, nthreads, t);
     block_sum<6>(t, smem, nthreads);
     if (threadIdx.x != 0) return;
-    tail_record(a, step, force_used, mode, a.plane_sums, t);
+    tail_record<FUSED>(a, step, force_used, mode, a.plane_sums, t);
     if (mode == 0) *a.step_ctr = step + 1;
 }
 
@@ -358,6 +366,7 @@ static __device__ __forceinline__ void step_tail(const StepArgs &a, long long st
 // block waits for another: the last arrival does the work, found with atomic
 // tickets.  `slot` numbers the block among the `ncontrib` contributors of
 // the plane; the call is block-uniform.
+template <bool RING, bool FUSED>
 __device__ __forceinline__ void plane_contribute(const StepArgs &a, double (&acc)[NP], int z, int slot, int ncontrib,
                                                  long long step, double force_used, int mode, int nthreads)
 {
@@ -394,18 +403,19 @@ __device__ __forceinline__ void plane_contribute(const StepArgs &a, double (&acc
     group_sync(nthreads);
     if (ticket != (unsigned)a.nz - 1) return;
     __threadfence();
-    if (a.tail) step_tail(a, step, force_used, mode, smem, nthreads);
+    if (a.tail) step_tail<RING, FUSED>(a, step, force_used, mode, smem, nthreads);
     if (threadIdx.x == 0) *a.total_ctr = 0;
     group_sync(nthreads);
 }
 
 // Epilogue of the scalar kernels: one block per (x-chunk, row-chunk) of a
 // plane, blockIdx.z = plane.
+template <bool RING, bool FUSED>
 __device__ __forceinline__ void block_epilogue(const StepArgs &a, double (&acc)[NP], long long step, double force_used,
                                                int mode)
 {
     const int bpp = gridDim.x * gridDim.y;
-    plane_contribute(a, acc, blockIdx.z, blockIdx.y * gridDim.x + blockIdx.x, bpp, step, force_used, mode, blockDim.x);
+    plane_contribute<RING, FUSED>(a, acc, blockIdx.z, blockIdx.y * gridDim.x + blockIdx.x, bpp, step, force_used, mode, blockDim.x);
 }
 
 }  // namespace dnslbm

@@ -29,9 +29,9 @@ __global__ void __launch_bounds__(128, 4) step_f64_kernel(const StepArgs p)
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int z = blockIdx.z;
     const int wall = plane_wall(p, z);
-    const double c0 = shift_entry(p, step)[z * 3 + 0];
-    const double c1 = shift_entry(p, step)[z * 3 + 1];
-    const double c2 = shift_entry(p, step)[z * 3 + 2];
+    const double c0 = shift_entry<false>(p, step)[z * 3 + 0];
+    const double c1 = shift_entry<false>(p, step)[z * 3 + 1];
+    const double c2 = shift_entry<false>(p, step)[z * 3 + 2];
     double acc[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) acc[i] = 0.0;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128, 4) step_f64_kernel(const StepArgs p)
             }
         }
     }
-    block_epilogue(p, acc, step, G, 0);
+    block_epilogue<false, false>(p, acc, step, G, 0);
 }
 
 // Reader-only reduction of the current state (after a load/init): force and
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(128) reduce_f64_kernel(const StepArgs p)
             acc[4] += jz / dens;
         }
     }
-    block_epilogue(p, acc, step, 0.0, 1);
+    block_epilogue<true, false>(p, acc, step, 0.0, 1);
 }
 
 // The same for a state left by an odd number of steps (post-collision
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(128) reduce_f64_odd_kernel(const StepArgs p)
             acc[4] += jz / dens;
         }
     }
-    block_epilogue(p, acc, step, 0.0, 1);
+    block_epilogue<true, false>(p, acc, step, 0.0, 1);
 }
 
 void launch_step_f64(const StepArgs &p, dim3 grid, dim3 block, bool odd, int tex, cudaStream_t s)
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256) slab_tail_kernel(const StepArgs a, int mo
     __shared__ double smem[32 * NP];
     const long long step = __ldcg(a.step_ctr);
     const double force_used = __ldcg(a.force + (step & 1));
-    step_tail(a, step, force_used, mode, smem, blockDim.x);
+    step_tail<false, false>(a, step, force_used, mode, smem, blockDim.x);
     __syncthreads();
     const int par = (int)((mode == 0 ? step + 1 : step) & 1);
     const double *src = a.shift + (size_t)par * a.nz * 3 + (size_t)z0 * 3;

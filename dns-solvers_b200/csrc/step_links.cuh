@@ -291,7 +291,7 @@ __device__ __forceinline__ void links_pass_body(const LinksLaunch &L, int blk)
             for (int i = 0; i < NP; ++i) acc[i] += (double)racc[i];
         }
     }
-    plane_contribute(p, acc, z, r, per_plane, step, G, 0, blockDim.x);
+    plane_contribute<true, !std::is_same<T, double>::value>(p, acc, z, r, per_plane, step, G, 0, blockDim.x);
 }
 
 constexpr int kLinksThreads = 128;

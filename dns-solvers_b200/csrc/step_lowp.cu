@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128, 4) step_lp_kernel(const StepArgs p)
             }
         }
     }
-    block_epilogue(p, acc, step, Gd, 0);
+    block_epilogue<true, true>(p, acc, step, Gd, 0);
 }
 
 template <typename T>
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(128) reduce_lp_kernel(const StepArgs p)
             acc[4] += (double)jz / rho;
         }
     }
-    block_epilogue(p, acc, step, 0.0, 1);
+    block_epilogue<true, true>(p, acc, step, 0.0, 1);
 }
 
 template <typename T>

@@ -584,7 +584,7 @@ __device__ __forceinline__ void flow_plane_done(const PersistArgs &a, const Chan
         }
         warp_sum<2>(f);
         if (lane == 0) {
-            p.force[(abs_step + 1) & 1] = tail_force(p, f[0], f[1]);
+            p.force[(abs_step + 1) & 1] = tail_force<false>(p, f[0], f[1]);
             st_release(L.force_ctr, abs_step + 1);
         }
     }
@@ -593,7 +593,7 @@ __device__ __forceinline__ void flow_plane_done(const PersistArgs &a, const Chan
     warp_sum<6>(t);
     __syncwarp();
     if (lane == 0) {
-        tail_record(p, abs_step, p.const_q ? __ldcg(p.force + (abs_step & 1)) : p.gx, 0, sums, t, !p.const_q);
+        tail_record<false>(p, abs_step, p.const_q ? __ldcg(p.force + (abs_step & 1)) : p.gx, 0, sums, t, !p.const_q);
         L.ftotal[ring] = 0;
     }
     __threadfence();

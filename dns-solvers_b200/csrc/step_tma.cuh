@@ -753,7 +753,8 @@ __device__ __forceinline__ void tma_step_body(const StepArgs &p, const TmaArgs &
             const int pi = gi / t.gpp;  // position of plane z in the kernel's plane list
             const int bfirst = (pi * t.gpp) / G_;
             const int blast = min(((pi + 1) * t.gpp - 1) / G_, (t.ngroups - 1) / G_);
-            plane_contribute(p, acc, z, blk - bfirst, blast - bfirst + 1, step, G, 0, nc);
+            plane_contribute<true, !std::is_same<T, double>::value>(p, acc, z, blk - bfirst, blast - bfirst + 1, step, G, 0,
+                                                                    nc);
 #pragma unroll
             for (int q = 0; q < NP; ++q) acc[q] = 0.0;
         }
