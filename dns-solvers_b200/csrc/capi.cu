@@ -602,11 +602,9 @@ static int create_ctx(const dnslbm_deck *deck, int slab, int z0, int nzs, Rows r
             // 628 -> 640 cells 1918 / 1966, 404 -> 416 580 / 734, 204 -> 208
             // 60.9 / 70.9, 92 -> 96 (7 -> 6 rows) 64.3 / 69.0, but 212 -> 216
             // (3 -> 2 rows) 164 / 151; FP32 204 -> 208 30.1 / 31.9, 628 -> 640
-            // 927 / 925, but 404 -> 416 244 / 240 (with riblets 260 / 264) and
-            // 644 -> 672 (2 -> 1 rows) 584 / 452: FP32 without solids in the
-            // flow stops at 2 % more bytes, the others at 5 %.
-            const bool tight = c->esize == 4 && deck->bc_mode != DNSLBM_BC_GENERAL;
-            const size_t row0 = (size_t)c->pitch * c->esize, most = row0 + row0 / (tight ? 50 : 20);
+            // 927 / 925, 404 -> 416 244 / 240 (with riblets 260 / 264,
+            // autotuned 274 / 307), but 644 -> 672 (2 -> 1 rows) 584 / 452.
+            const size_t row0 = (size_t)c->pitch * c->esize, most = row0 + row0 / 20;
             size_t row = row0;
             while (row <= most && !tensor_rows(row, default_rows(c, row))) row += 16;
             if (row <= most && 4 * default_rows(c, row) >= 3 * default_rows(c, row0)) c->pitch = (int)(row / c->esize);
