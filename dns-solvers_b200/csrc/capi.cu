@@ -2058,6 +2058,7 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
     int ncand = 0;
     double best_ms = 1e30;
     const TmaChoice own = save_choice(c);
+    const bool uses_flow_shape = uses_flow(c);
     TmaChoice best = own;
     int rc;
     // the per-thread kernel
@@ -2093,6 +2094,14 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
     auto configure = [&](int k, int st, int cons, int bps, int seg) {
         return tma_configure(c, k, st, cons, bps, seg) || (uses_flow(c) && flow_reserve(c));
     };
+    // the shape the context has (the default rows per stage are any number up
+    // to 8)
+    if (own.use_tma && own.t.k > 0) {
+        const int cons = own.threads - (uses_flow_shape ? 64 : 32);
+        if (!configure(own.t.k, own.t.stages, cons, 0, own.t.nseg > 1 ? own.t.seg : 0) &&
+            (rc = timed(own.t.k, own.t.stages, own.t.nseg > 1 ? own.t.seg : 0, cons)))
+            return rc;
+    }
     // the default consumer count and the widest consumer sets (a block with
     // large stages is alone on its SM and needs more warps)
     const int widest = std::min(352, (c->nx + 31) / 32 * 32 + 32);
