@@ -609,57 +609,68 @@ __device__ __forceinline__ void flow_stores(const PersistArgs &a, const FlowTabl
     volatile int *s_abort = sm.abort;
     // the group whose stores were committed last, not yet announced
     bool pend = false;
-    unsigned *pflag = nullptr, *pcount = nullptr, pstep = 0;
+    int pz = 0, pg = 0, pstep = 0;
+    long long pabs = 0;
+    unsigned *pflag = nullptr, *pcount = nullptr;
+    // where it is announced: for one channel worked out then, which is off the
+    // path of the stage; a batch's entry is gone by then
+    auto address = [&](const ChannelLaunch &L) {
+        pflag = L.flags + (size_t)pz * L.t.gpp + pg;
+        pcount = L.fctr + (size_t)(pabs & (L.p.ring - 1)) * L.p.nz + pz;
+    };
     // raise its flag (its copies have landed) and count it in its plane,
     // without waiting for either
     auto announce = [&]() {
+        if (ONE) address(chans.at(0));
         if (lane < Q) fence_async_global();
         __syncwarp();
         if (lane == 0) {
             __threadfence();
-            *reinterpret_cast<volatile unsigned *>(pflag) = pstep + 1u;
+            *reinterpret_cast<volatile unsigned *>(pflag) = (unsigned)pstep + 1u;
             asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(pcount) : "memory");
         }
     };
     // The plane to look after.  (The warp that counts a plane's last group
     // could sum it instead, but then every count needs its answer, and the sum
     // delays that block's stores: 628x314x200 FP64 7 % slower.)
-    int dc = -1, ds = 0, dz = 0;
-    unsigned dfirst = 0, dn = 0;  // place in the sequence of channel dc's first plane, its (step, plane) pairs
-    bool dfree = false;           // the counter of the plane is this step's
-    long long dabs = 0;
-    const unsigned *dcount = nullptr;
+    // One plane at a time, and none beside it: a warp in a step's tail waits for
+    // the tail before, whose planes are all counted and each held by a warp
+    // that holds no other, so nobody waits in a circle.  (With the next plane
+    // taken ahead a batch of 450 channels ran into the wait limit: a warp's
+    // first plane lacked a group whose block waited for the second.)
+    int dc = 0, ds = 0, dz = 0;
+    unsigned dfirst = 0;  // place in the sequence of channel dc's first plane
+    bool dfree = false;   // the counter of the plane is this step's
+    int dcopy = -1;       // channel of the copy
     auto take_duty = [&]() {
         unsigned d = 0;
         if (lane == 0) d = atomicAdd(a.counter + 1, 1u);
         d = __shfl_sync(0xffffffffu, d, 0);
-        if (d - dfirst >= dn) {
-            do {
-                dfirst += dn;
-                if (++dc >= chans.count()) return;
-                dn = (unsigned)chans.entry(dc).p.nz * (unsigned)a.nsteps;
-            } while (d - dfirst >= dn);
-            chans.fetch(1, dc, lane);
+        for (; dc < chans.count(); ++dc) {
+            const unsigned nz = (unsigned)chans.entry(dc).p.nz, n = nz * (unsigned)a.nsteps;
+            if (d - dfirst < n) {
+                ds = (int)((d - dfirst) / nz);
+                dz = (int)(d - dfirst - (unsigned)ds * nz);
+                break;
+            }
+            dfirst += n;
         }
-        const ChannelLaunch &L = chans.duty();
-        ds = (int)((d - dfirst) / (unsigned)L.p.nz);
-        dz = (int)(d - dfirst) - ds * L.p.nz;
-        dabs = __ldcg(L.base) + ds;
-        dcount = L.fctr + (size_t)(dabs & (L.p.ring - 1)) * L.p.nz + dz;
-        dfree = ds < L.p.ring;
+        if (!ONE && dc < chans.count() && dc != dcopy) chans.fetch(1, dcopy = dc, lane);
+        dfree = false;
     };
     take_duty();
     // true: the plane is done, and the next one taken
     auto service = [&]() {
         if (dc >= chans.count()) return false;
         const ChannelLaunch &L = chans.duty();
+        const long long abs_step = __ldcg(L.base) + ds;
         if (!dfree) {  // the step that had the counter before has cleared it when it is logged
-            if (!__all_sync(0xffffffffu, ld_acquire(L.p.step_ctr) > dabs - L.p.ring)) return false;
+            if (!__all_sync(0xffffffffu, ds < L.p.ring || ld_acquire(L.p.step_ctr) > abs_step - L.p.ring)) return false;
             dfree = true;
         }
-        const unsigned n = ld_acquire(dcount);
+        const unsigned n = ld_acquire(L.fctr + (size_t)(abs_step & (L.p.ring - 1)) * L.p.nz + dz);
         if (!__all_sync(0xffffffffu, n == (unsigned)L.t.gpp)) return false;
-        flow_plane_done(a, L, dabs, dz, lane, s_abort);
+        flow_plane_done(a, L, abs_step, dz, lane, s_abort);
         take_duty();
         return true;
     };
@@ -723,12 +734,14 @@ __device__ __forceinline__ void flow_stores(const PersistArgs &a, const FlowTabl
             for (int q = lane >> 3; q < nwarps; q += 4) s += w[q * NP];
             s += __shfl_xor_sync(0xffffffffu, s, 8);
             s += __shfl_xor_sync(0xffffffffu, s, 16);
-            const size_t plane = (size_t)(habs & (L.p.ring - 1)) * L.p.nz + hz;
-            if (lane < NP) L.fpart[(plane * L.t.gpp + hg) * NP + lane] = s;
-            pflag = L.flags + (size_t)hz * L.t.gpp + hg;
-            pcount = L.fctr + plane;
-            pstep = (unsigned)hs;
+            const int ring = (int)(habs & (L.p.ring - 1));
+            if (lane < NP) L.fpart[(((size_t)ring * L.p.nz + hz) * L.t.gpp + hg) * NP + lane] = s;
         }
+        pz = hz;
+        pg = hg;
+        pstep = hs;
+        pabs = habs;
+        if (!ONE) address(L);
         bulk_wait_read_all();  // the stores have read the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(sm.freed + st);
