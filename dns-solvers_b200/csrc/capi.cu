@@ -2094,14 +2094,6 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
     auto configure = [&](int k, int st, int cons, int bps, int seg) {
         return tma_configure(c, k, st, cons, bps, seg) || (uses_flow(c) && flow_reserve(c));
     };
-    // the shape the context has (the default rows per stage are any number up
-    // to 8)
-    if (own.use_tma && own.t.k > 0) {
-        const int cons = own.threads - (uses_flow_shape ? 64 : 32);
-        if (!configure(own.t.k, own.t.stages, cons, 0, own.t.nseg > 1 ? own.t.seg : 0) &&
-            (rc = timed(own.t.k, own.t.stages, own.t.nseg > 1 ? own.t.seg : 0, cons)))
-            return rc;
-    }
     // the default consumer count and the widest consumer sets (a block with
     // large stages is alone on its SM and needs more warps)
     const int widest = std::min(352, (c->nx + 31) / 32 * 32 + 32);
@@ -2143,6 +2135,14 @@ extern "C" int dnslbm_autotune(dnslbm_ctx *c, int steps, char *report, size_t re
             if (configure(b0.k, b0.st, b0.cons, bps, b0.seg)) continue;
             if ((rc = timed(b0.k, b0.st, b0.seg, b0.cons))) return rc;
         }
+    }
+    // the shape the context has (the default rows per stage are any number up
+    // to 8), last: the searches above go on from the best of their own grid
+    if (own.use_tma && own.t.k > 0) {
+        const int cons = own.threads - (uses_flow_shape ? 64 : 32);
+        if (!configure(own.t.k, own.t.stages, cons, 0, own.t.nseg > 1 ? own.t.seg : 0) &&
+            (rc = timed(own.t.k, own.t.stages, own.t.nseg > 1 ? own.t.seg : 0, cons)))
+            return rc;
     }
     if (bt.k > 0 && bt.ms < best_ms) best_ms = bt.ms, best = bt.ch;  // one shape for both parities
     const bool per_step = c->slab || ordered_sums(c->deck);
