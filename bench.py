@@ -13,8 +13,11 @@ between timed steps.
 
 One JSON line (rank 0):
   value       MLUPS of the FP64 kernel, inputs resident in HBM, CUDA events
-  roofline    dominant step kernel: algorithmic bytes (2 x 19 x 8 B per cell)
-              / mean launch time, against the measured HBM copy bandwidth
+  roofline    step kernel: algorithmic bytes (2 x 19 x 8 B per cell) / time per
+              step of the timed steps (persistent kernel; mean launch time of
+              the slower parity for a kernel of one launch per step), against
+              the measured HBM copy bandwidth.  Two steps at once find part of
+              the bytes in L2: traffic gives the DRAM bytes per step
   variants    the same workload with FP32 / FP16 deviation storage: MLUPS,
               roofline fraction and error against the FP64 run (which is
               bit-identical to the CPU oracle, see tests/test_gpu_parity.py)
@@ -73,8 +76,9 @@ def hbm_peak():
         return FALLBACK_HBM_GBS, "fallback"
 
 
-def ncu_traffic(kernel_key):
-    """DRAM bytes per launch from the committed ncu summary, if any."""
+def ncu_traffic(workload, precision, kernel):
+    """DRAM bytes per step of a kernel from the committed ncu summary, if any."""
+    kernel_key = f"{workload}:f{precision}:{kernel.split('<')[0]}"
     p = os.path.join(ROOT, "profiles", "traffic.json")
     try:
         with open(p) as f:
@@ -263,6 +267,26 @@ def parity_fracs(bpc, cells, ms_even, ms_odd, n_even, n_odd, peak):
     return frac(ms_even, n_even), frac(ms_odd, n_odd)
 
 
+def roofline(bpc, cells, peak, kdesc, ms_per_step, ms_even, ms_odd, n_even, n_odd):
+    """Achieved algorithmic bytes of the step kernel against the copy
+    bandwidth: of the timed steps for the persistent kernel, whose steps
+    overlap; of the parity with the larger summed device time otherwise."""
+    kname, launch_ms = kdesc.split(" ")[0], ms_per_step
+    if "persist_batch_kernel" in kdesc:
+        of = "the timed steps; frac_even and frac_odd: a second run of one step per launch, which the time loop does not use"
+    else:
+        of = "a second run of K steps with a CUDA event pair around every launch"
+        odd = ms_odd >= ms_even
+        kname += " (odd parity)" if odd else " (even parity)"
+        launch_ms = ms_odd / n_odd if odd else ms_even / n_even
+    achieved = bpc * cells / (launch_ms / 1e3) / 1e9
+    fe, fo = parity_fracs(bpc, cells, ms_even, ms_odd, n_even, n_odd, peak)
+    return {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
+            "kernel": kname, "kernel_config": kdesc, "launch_ms": round(launch_ms, 4), "launch_ms_from": of,
+            "frac_even": fe, "frac_odd": fo, "whole_step_frac": round(bpc * cells / (ms_per_step / 1e3) / 1e9 / peak, 4),
+            "algorithmic_bytes_per_launch": bpc * cells, "bytes_per_cell": bpc}
+
+
 def variant_summary(v):
     r, e = v["roofline"], v["error_vs_f64"]
     return {"value": v["value"], "unit": "MLUPS", "ms_per_step": v["ms_per_step"], "speedup_vs_f64": v["speedup_vs_f64"],
@@ -400,24 +424,10 @@ def run_ours(args):
     n_odd = args.steps - n_even
     value = d.world * cells * args.steps / (tmax / 1e3) / 1e6
     bpc = ch.bytes_per_cell
-    # dominant kernel: the parity with the larger summed device time
     kdesc = ch.kernel
-    kbase = kdesc.split(" ")[0]
-    if odd >= even:
-        kname, kms, kn = kbase + " (odd parity)", odd, n_odd
-    else:
-        kname, kms, kn = kbase + " (even parity)", even, n_even
-    launch_s = kms / kn / 1e3
-    achieved = bpc * cells / launch_s / 1e9
-    traffic = ncu_traffic(f"{wl.name}:f{args.precision}")
-    fe, fo = parity_fracs(bpc, cells, even, odd, n_even, n_odd, peak)
-    roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": f"{peak_src} (MEASURED_PEAKS.json)",
-            "kernel": kname, "kernel_config": kdesc, "autotune": tune, "launch_ms": round(launch_s * 1e3, 4),
-            "launch_ms_from": "a second run of K steps with a CUDA event pair around every launch",
-            "frac_even": fe, "frac_odd": fo,
-            "whole_step_frac": round(bpc * cells / (tmax / args.steps / 1e3) / 1e9 / peak, 4),
-            "algorithmic_bytes_per_launch": bpc * cells, "bytes_per_cell": bpc}
+    roof = roofline(bpc, cells, peak, kdesc, tmax / args.steps, even, odd, n_even, n_odd)
+    roof.update(traffic=ncu_traffic(wl.name, args.precision, kdesc), peak_source=f"{peak_src} (MEASURED_PEAKS.json)",
+                autotune=tune)
 
     variants = {}
     if not args.no_variants and args.precision == 64:
@@ -437,19 +447,14 @@ def run_ours(args):
             st = c2.statistics()
             vel, _ = c2.moments()
             b2 = c2.bytes_per_cell
-            k2 = max(e2, o2) / (n_odd if o2 >= e2 else n_even) / 1e3
-            ach2 = b2 * cells / k2 / 1e9
-            fe2, fo2 = parity_fracs(b2, cells, e2, o2, n_even, n_odd, peak)
+            roof2 = roofline(b2, cells, peak, c2.kernel, t2 / args.steps, e2, o2, n_even, n_odd)
+            roof2.update(traffic=ncu_traffic(wl.name, prec, c2.kernel), autotune=tune2)
             um_ref, um = ref_stats[0, 1:-1], st[0, 1:-1]
             urms_ref, urms = ref_stats[3, 1:-1], st[3, 1:-1]
             variants[f"f{prec}"] = {
                 "value": round(cells * args.steps / (t2 / 1e3) / 1e6, 1), "unit": "MLUPS",
                 "ms_per_step": round(t2 / args.steps, 4), "speedup_vs_f64": round(tot / t2, 3),
-                "roofline": {"bound": "hbm", "achieved": round(ach2, 1), "peak": peak, "unit": "GB/s",
-                             "frac": round(ach2 / peak, 4), "frac_even": fe2, "frac_odd": fo2, "bytes_per_cell": b2,
-                             "whole_step_frac": round(b2 * cells / (t2 / args.steps / 1e3) / 1e9 / peak, 4),
-                             "traffic": ncu_traffic(f"{wl.name}:f{prec}"), "kernel_config": c2.kernel,
-                             "autotune": tune2},
+                "roofline": roof2,
                 "error_vs_f64": {
                     "after_steps": done,
                     "mean_u_profile_max_rel": float(np.max(np.abs(um - um_ref)) / np.max(np.abs(um_ref))),

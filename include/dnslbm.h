@@ -340,8 +340,10 @@ void dnslbm_host_free(void *ptr);
  * state and logs) advanced together by one persistent kernel: one launch
  * runs a chunk of 32 steps (the time loop, replayed from a CUDA graph), its
  * blocks taking row groups in sequence, channel after channel; a group
- * starts when the groups around it are done with the step before.  All decks
- * share one precision and device.  Use dnslbm_batch_channel(b, i) with the
+ * starts when the groups around it are done with the step before.  (FP32 or
+ * FP16 with some channel at a constant flow rate: a cooperative launch whose
+ * sums go by runs of rows, so that results keep their roundings.)  All decks
+ * share one precision and device.  Any number of channels.  Use dnslbm_batch_channel(b, i) with the
  * single-channel calls (flags, load/store, logs, statistics) between batch
  * steps.  The environment variable DNSLBM_BATCH=launch selects one launch
  * per step instead.  No counterpart in the reference (one channel per run). */
